@@ -290,7 +290,10 @@ int zsme_batch_get_time(zsme_handle* h, int32_t i, double* t, double* dt);
  * in device memory; 64..1024 runs them as one kernel over tiles of
  * consecutive cells evaluating at most that many faces each, the
  * contributions kept in shared memory (the face block size and cap apply);
- * fuse_final: 1 lets the finalize kernel form the last SSP stage's result
+ * fuse_final: with tiles (and positivity "none") 1 forms the face states too
+ * inside that kernel, a whole stage or right-hand side per launch, with
+ * prep_lean 0..1, 2 or 3..4 as 1, 2 or 4 threads per cell and block sizes and
+ * caps of its own (the configuration a new handle has); without tiles 1 lets the finalize kernel form the last SSP stage's result
  * itself from the face contributions (separate face and gather kernels,
  * order 2, positivity other than "mood"), so that result never round-trips
  * through device memory; prep_lean: 1 (default) forms the order-2 face

@@ -15,76 +15,80 @@
 
 namespace zsme {
 
-// One face's contributions (TransportStep.hpp:420-552): out[r * ostride] for
+// One face's contributions (TransportStep.hpp:420-552) from its reconstructed
+// states, variable r of side d at fs[(d NQ + r) * fstride]: out[r * ostride] for
 // r in [0, NQ) the fluctuation into the left cell, [NQ, 2 NQ) into the right
 // cell (interior faces only), [2 NQ, 3 NQ) the flux, each times the area.
-// Returns false, writing nothing, for an exterior face without a condition
-// (no flux) and for a face of an inactive instance.
+// fs and out may be the same row (stage_kernel): every state is read before
+// the first contribution is written.  Returns false, writing nothing, for an
+// exterior face without a condition (no flux) and for a face of an inactive
+// instance.
+struct FaceGeom {
+    int f, L, R, bc, I;
+    double area, nx, ny;
+    __device__ __forceinline__ void load(const MeshDev& m, int face) {
+        f = face;
+        I = face_instance(m, f);
+        L = m.face_L[f];
+        R = m.face_R[f];
+        bc = m.face_bc[f];
+        area = m.farea[f];
+        nx = m.fn[f];
+        ny = m.fn[m.F + f];
+    }
+};
+
 template <class M, class N>
-__device__ __forceinline__ bool face_contrib(const MeshDev& m, int f, const double* __restrict__ fs,
+__device__ __forceinline__ bool face_contrib(const MeshDev& m, const FaceGeom& fg, const double* fs, size_t fstride,
                                              const double* __restrict__ aux, const double* __restrict__ params,
                                              double t_host, const double* t_dev, double stage_frac,
                                              const double* __restrict__ dt_step, const int* __restrict__ active,
-                                             double* __restrict__ out, size_t ostride) {
+                                             double* out, size_t ostride) {
     constexpr int NQ = M::n_dof_q, NA = M::n_dof_qaux;
     const int F = m.F, C = m.C;
-    const int I = face_instance(m, f);
+    const int f = fg.f, I = fg.I, L = fg.L, R = fg.R, bc = fg.bc;
     if (active && !active[I]) return false;
     const double* p = params + (size_t)I * m.np;
-    const int R = m.face_R[f];
-    const int bc = m.face_bc[f];
     if (R < 0 && bc < 0) return false;  // exterior face without a condition: no flux
-    const int L = m.face_L[f];
-    // stage time t0 + dt * i/(s-1) (only time-dependent BCs / aux see it)
-    const double t = t_dev ? (t_dev[I] + stage_frac * (dt_step ? dt_step[I] : 0.0)) : t_host;
-    const double area = m.farea[f];
-    const double nh[3] = {m.fn[f], m.fn[F + f], 0.0};
+    const double area = fg.area;
+    const double nh[3] = {fg.nx, fg.ny, 0.0};
     const double xf[3] = {m.fc[f], m.fc[F + f], 0.0};
-    double qL[NQ], aLc[NA];
+    double qL[NQ], qR[NQ], aLc[NA], aL[NA], aR[NA];
 #pragma unroll
-    for (int i = 0; i < NQ; ++i) qL[i] = fs[(size_t)i * F + f];
+    for (int i = 0; i < NQ; ++i) qL[i] = fs[i * fstride];
 #pragma unroll
     for (int i = 0; i < NA; ++i) aLc[i] = aux[(size_t)i * C + L];
-    double aL[NA], aR[NA];
     if (R >= 0) {
-        double qR[NQ], aRc[NA];
+        double aRc[NA];
 #pragma unroll
-        for (int i = 0; i < NQ; ++i) qR[i] = fs[((size_t)NQ + i) * F + f];
+        for (int i = 0; i < NQ; ++i) qR[i] = fs[(NQ + i) * fstride];
 #pragma unroll
         for (int i = 0; i < NA; ++i) aRc[i] = aux[(size_t)i * C + R];
-        {
-            auto ra = M::update_aux_variables(qL, aLc, p, 0.0, xf);
-            auto rb = M::update_aux_variables(qR, aRc, p, 0.0, xf);
+        auto ra = M::update_aux_variables(qL, aLc, p, 0.0, xf);
+        auto rb = M::update_aux_variables(qR, aRc, p, 0.0, xf);
 #pragma unroll
-            for (int i = 0; i < NA; ++i) { aL[i] = ra[i]; aR[i] = rb[i]; }
-        }
-        const auto flux = N::numerical_flux(qL, qR, aL, aR, p, nh);
-        const auto nc = N::numerical_fluctuations(qL, qR, aL, aR, p, nh);
-#pragma unroll
-        for (int i = 0; i < NQ; ++i) {
-            out[i * ostride] = nc[NQ + i] * area;
-            out[(NQ + i) * ostride] = nc[i] * area;
-            out[(2 * NQ + i) * ostride] = flux[i] * area;
-        }
+        for (int i = 0; i < NA; ++i) { aL[i] = ra[i]; aR[i] = rb[i]; }
     } else {
-        {
-            auto ra = M::update_aux_variables(qL, aLc, p, t, xf);
+        // stage time t0 + dt * i/(s-1) (only time-dependent BCs / aux see it)
+        const double t = t_dev ? (t_dev[I] + stage_frac * (dt_step ? dt_step[I] : 0.0)) : t_host;
+        auto ra = M::update_aux_variables(qL, aLc, p, t, xf);
 #pragma unroll
-            for (int i = 0; i < NA; ++i) aL[i] = ra[i];
-        }
-        const auto qR = M::boundary_conditions(bc, qL, aL, p, nh, xf, t, 0.0);
-        {
-            auto rb = M::update_aux_variables(qR.data, aL, p, t, xf);
+        for (int i = 0; i < NA; ++i) aL[i] = ra[i];
+        const auto qb = M::boundary_conditions(bc, qL, aL, p, nh, xf, t, 0.0);
 #pragma unroll
-            for (int i = 0; i < NA; ++i) aR[i] = rb[i];
-        }
-        const auto flux = N::numerical_flux(qL, qR.data, aL, aR, p, nh);
-        const auto nc = N::numerical_fluctuations(qL, qR.data, aL, aR, p, nh);
+        for (int i = 0; i < NQ; ++i) qR[i] = qb[i];
+        auto rb = M::update_aux_variables(qR, aL, p, t, xf);
 #pragma unroll
-        for (int i = 0; i < NQ; ++i) {
-            out[i * ostride] = nc[NQ + i] * area;
-            out[(2 * NQ + i) * ostride] = flux[i] * area;
-        }
+        for (int i = 0; i < NA; ++i) aR[i] = rb[i];
+    }
+    // one copy of the plugin's functions serves both kinds of face
+    const auto flux = N::numerical_flux(qL, qR, aL, aR, p, nh);
+    const auto nc = N::numerical_fluctuations(qL, qR, aL, aR, p, nh);
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+        out[i * ostride] = nc[NQ + i] * area;
+        if (R >= 0) out[(NQ + i) * ostride] = nc[i] * area;
+        out[(2 * NQ + i) * ostride] = flux[i] * area;
     }
     return true;
 }
@@ -101,7 +105,10 @@ __global__ void __launch_bounds__(128, MINB) face_kernel(MeshDev m, int f0, int 
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= fcount) return;
     const int f = f0 + r;
-    face_contrib<M, N>(m, f, fs, aux, params, t_host, t_dev, stage_frac, dt_step, active, fb + f, (size_t)m.F);
+    FaceGeom fg;
+    fg.load(m, f);
+    face_contrib<M, N>(m, fg, fs + f, (size_t)m.F, aux, params, t_host, t_dev, stage_frac, dt_step, active, fb + f,
+                       (size_t)m.F);
 }
 
 // Division by the volume (TransportStep.hpp:555-560) and the SSP-RK(s,2)
@@ -297,8 +304,10 @@ __global__ void __launch_bounds__(128, MINB) flux_tile_kernel(MeshDev m, Opts o,
     const int st = tl.stride;
     for (int lf = threadIdx.x; lf < nf; lf += blockDim.x) {
         const int f = lf < nown ? f0 + lf : tl.in_faces[i0 + lf - nown];
-        face_contrib<M, N>(m, f, fs, aux, params, t_host, t_dev, stage_frac, dt_step, active, rows + lf,
-                           (size_t)st);
+        FaceGeom fg;
+        fg.load(m, f);
+        face_contrib<M, N>(m, fg, fs + f, (size_t)m.F, aux, params, t_host, t_dev, stage_frac, dt_step, active,
+                           rows + lf, (size_t)st);
     }
     __syncthreads();
     const int C = m.C, K = m.K;

@@ -64,7 +64,7 @@ bool solve_spd(int n, std::vector<double>& a, std::vector<double>& b) {
 
 }  // namespace
 
-int prepare_mesh(const zsme_mesh& m, PreparedMesh& out) {
+int prepare_mesh(const zsme_mesh& m, PreparedMesh& out, bool least_squares) {
     const int C = m.n_cells, F = m.n_faces, K = m.max_faces, D = m.dim;
     if (C <= 0 || F <= 0) return set_error(ZSME_ERR_MESH, "empty mesh");
     if (K < 1 || K > 4) return set_error(ZSME_ERR_MESH, "max_faces must be in [1, 4]");
@@ -204,7 +204,7 @@ int prepare_mesh(const zsme_mesh& m, PreparedMesh& out) {
             }
             const double dist = std::sqrt(d2);
             if (dist < p.rc[c]) p.rc[c] = dist;
-            if (other >= 0) {
+            if (other >= 0 && least_squares) {
                 if (std::find(nb_cell.begin(), nb_cell.end(), other) != nb_cell.end()) continue;
                 nb_cell.push_back(other);
                 nb_slot.push_back(k);
@@ -317,6 +317,82 @@ int build_tiles(const PreparedMesh& p, int max_faces, FaceTiles& t) {
         t.n++;
     }
     if (f0 != F) return set_error(ZSME_ERR_MESH, "tiles do not cover the faces");
+    return ZSME_OK;
+}
+
+int build_stage_tiles(const PreparedMesh& p, const FaceTiles& t, int order, bool green_gauss, StageTiles& s) {
+    const int C = p.C, K = p.K, n = t.n;
+    s = StageTiles();
+    s.ext_off.assign(n + 1, 0);
+    s.gho_off.assign(n + 1, 0);
+    s.ent_off.assign(n + 1, 0);
+    s.ring1.assign(n, 0);
+    std::vector<int> stamp(C, -1), local(C, 0), fstamp(p.F, -1), frow(p.F, 0);
+    // first pass: the rings
+    for (int b = 0; b < n; ++b) {
+        const int c0 = t.cell_off[b], c1 = t.cell_off[b + 1];
+        const int e0 = (int)s.ext_cell.size();
+        for (int c = c0; c < c1; ++c) stamp[c] = b;
+        auto ring = [&](int c) {
+            for (int k = 0; k < K; ++k) {
+                const int nb = p.slot_nbr[(size_t)k * C + c];
+                if (nb >= 0 && stamp[nb] != b) {
+                    stamp[nb] = b;
+                    s.ext_cell.push_back(nb);
+                }
+            }
+        };
+        for (int c = c0; c < c1; ++c) ring(c);
+        const int e1 = (int)s.ext_cell.size();
+        s.ring1[b] = e1 - e0;
+        if (order >= 2)
+            for (int e = e0; e < e1; ++e) ring(s.ext_cell[e]);
+        s.ext_off[b + 1] = (int)s.ext_cell.size();
+        s.ent_off[b + 1] = s.ent_off[b] + (c1 - c0) + s.ring1[b];
+    }
+    const size_t NE = s.ent_off[n];
+    s.loc.assign(K * NE, kLocNone | (kRowNone << 12));
+    std::fill(stamp.begin(), stamp.end(), -1);
+    s.fits = t.max_faces < (int)kRowNone;
+    for (int b = 0; b < n; ++b) {
+        const int c0 = t.cell_off[b], nc = t.cell_off[b + 1] - c0, e0 = s.ext_off[b], ne = s.ext_off[b + 1] - e0;
+        const int f0 = t.face_off[b], nown = t.face_off[b + 1] - f0;
+        for (int f = f0; f < f0 + nown; ++f) { fstamp[f] = b; frow[f] = f - f0; }
+        for (int i = t.in_off[b]; i < t.in_off[b + 1]; ++i) {
+            fstamp[t.in_faces[i]] = b;
+            frow[t.in_faces[i]] = nown + i - t.in_off[b];
+        }
+        for (int l = 0; l < nc + ne; ++l) {
+            const int c = l < nc ? c0 + l : s.ext_cell[e0 + l - nc];
+            stamp[c] = b;
+            local[c] = l;
+        }
+        int ghosts = 0;
+        for (int l = 0; l < nc + s.ring1[b]; ++l) {
+            const int c = l < nc ? c0 + l : s.ext_cell[e0 + l - nc];
+            const size_t ent = (size_t)s.ent_off[b] + l;
+            for (int j = 0; j < K; ++j) {
+                const int k = green_gauss ? (p.order[c] >> (2 * j)) & 3 : j;
+                const size_t q = (size_t)k * C + c;
+                const int f = p.slot_face[q];
+                if (f < 0) continue;
+                const int nb = p.slot_nbr[q], meta = p.slot_meta[q];
+                uint32_t across = kLocNone;
+                if (nb >= 0) {
+                    if (stamp[nb] == b) across = (uint32_t)local[nb];
+                } else if (((meta >> 3) - 2) >= 0 && green_gauss && order >= 2) {
+                    across = (uint32_t)(nc + ne + ghosts++);
+                    s.gho_cell.push_back(l);
+                    s.gho_face.push_back(f);
+                }
+                const uint32_t row = fstamp[f] == b ? (uint32_t)frow[f] : kRowNone;
+                s.loc[j * NE + ent] = across | (row << 12) | ((uint32_t)((meta >> 2) & 1) << 23) | ((uint32_t)k << 24);
+            }
+        }
+        s.gho_off[b + 1] = (int)s.gho_cell.size();
+        s.max_local = std::max(s.max_local, nc + ne + ghosts);
+    }
+    s.fits = s.fits && s.max_local < (int)kLocNone;
     return ZSME_OK;
 }
 

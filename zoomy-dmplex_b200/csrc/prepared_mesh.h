@@ -34,12 +34,15 @@ struct LaunchConfig {
     int prep, face, gather, finalize;  // threads per block
     int prep_occ = 1, face_occ = 1;    // register cap, blocks per SM: prep 1, 2, 3, 4, 6, 8; face 1-4
     int finalize_occ = 1;              // register cap of finalize, blocks of 128 per SM: 1-4
-    int tile_faces = 0;                // > 0: fused face + gather kernel over tiles of at most this many
-                                       // faces (64..1024); 0: separate face and gather kernels
-    int fuse_final = 0;                // 1: with separate face and gather kernels, the last stage's
-                                       // gather runs inside the finalize kernel
+    int tile_faces = 0;                // > 0: kernels over tiles of at most this many faces (64..1024):
+                                       // the whole stage in one (fuse_final = 1) or face + gather;
+                                       // 0: separate face and gather kernels
+    int fuse_final = 0;                // 1: with tiles, face states, fluxes and sums in one kernel per
+                                       // stage (stage_kernel); with separate kernels, the last
+                                       // stage's gather inside the finalize kernel
     int prep_lean = 1;                 // order-2 face states: prep_kernel (0), prep_lean_kernel (1),
-                                       // prep_split_kernel with 2..4 threads per cell
+                                       // prep_split_kernel with 2..4 threads per cell; stage_kernel's
+                                       // threads per cell: 1 (0, 1), 2, 4 (3, 4)
 };
 
 // Tiles of the fused face + gather kernel.  A tile is a run of consecutive
@@ -60,9 +63,32 @@ struct FaceTiles {
 };
 int build_tiles(const PreparedMesh& p, int max_faces, FaceTiles& out);
 
+// What the whole-stage kernel needs beside FaceTiles.  A tile's block holds
+// the stage state of its own cells (local indices 0 .. n), of the cells across
+// its faces (ring 1, whose face states towards the tile it reconstructs too)
+// and, at order 2, of the cells next to those (ring 2: values only), then one
+// ghost value per boundary face with a condition of the own and ring-1 cells
+// (Green-Gauss only).  "Entries" are the own and ring-1 cells, tile by tile.
+struct StageTiles {
+    bool fits = false;       // every local index fits the packed fields below
+    int max_local = 0;       // most cells + ghosts of one tile
+    std::vector<int> ext_off, ring1, ext_cell;   // [n + 1], [n], ring-1 then ring-2 cells
+    std::vector<int> gho_off, gho_cell, gho_face;  // [n + 1], local index of the cell, face
+    std::vector<int> ent_off;                    // [n + 1]
+    // [K][entries]: the entry's j-th face (increasing original face id for
+    // Green-Gauss, cone order for least squares), packed as below
+    std::vector<uint32_t> loc;
+};
+// loc: bits 0-11 local index across the face (kLocNone: none), bits 12-22 the
+// face's row in the tile (kRowNone: not one of the tile's faces), bit 23 the
+// entry is support[0], bits 24-25 the cell's slot of the face
+constexpr uint32_t kLocNone = 0xfff, kRowNone = 0x7ff;
+int build_stage_tiles(const PreparedMesh& p, const FaceTiles& t, int order, bool green_gauss, StageTiles& out);
+
 // Builds the layout (validates the connectivity; computes the least-squares
 // weights as LeastSquaresGradient::Setup does, Gradient.hpp:222-298).
-int prepare_mesh(const zsme_mesh& m, PreparedMesh& out);
+// least_squares = false leaves the weights zero.
+int prepare_mesh(const zsme_mesh& m, PreparedMesh& out, bool least_squares = true);
 // Concatenates prepared instances (same dim and K) into one layout.
 int concat_meshes(std::vector<PreparedMesh>& parts, PreparedMesh& out);
 

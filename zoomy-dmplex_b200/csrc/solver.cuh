@@ -18,6 +18,7 @@
 #include "step_kernels.cuh"
 #include "face_kernels.cuh"
 #include "source_kernels.cuh"
+#include "stage_kernel.cuh"
 #include "adjoint_kernels.cuh"
 #include "imex_kernels.cuh"
 #include "implicit_kernels.cuh"
@@ -107,6 +108,13 @@ class Solver final : public SolverBase {
     // tiles of the fused face + gather kernel (LaunchConfig::tile_faces > 0)
     DevBuf<int> tile_cell_off_, tile_face_off_, tile_in_off_, tile_in_faces_, tile_ord_lf_;
     int tile_n_ = 0, tile_stride_ = 0, tile_built_ = 0;  // tile_built_: the tile_faces they were built for
+    // the whole-stage kernel's view of the same tiles (LaunchConfig::fuse_final with tile_faces > 0)
+    DevBuf<StageTile> st_tile_;
+    DevBuf<int> st_ext_cell_, st_gho_cell_, st_gho_face_;
+    DevBuf<unsigned> st_loc_;
+    DevBuf<double> st_geo_;
+    int st_built_ = 0, st_entries_ = 0, st_fst_ = 0, st_cst_ = 0;
+    bool st_fits_ = false;
     bool ready_ = false;          // init done: mesh on the device
     bool lean_ok_ = false;        // 32-bit element offsets cover every array prep_lean_kernel indexes
     DerivSpecs deriv_{};          // derivative aux slots refreshed at every state update (n = 0: none)
@@ -240,10 +248,13 @@ class Solver final : public SolverBase {
     // (Re)builds the tiles for lc_.tile_faces; outside any stream capture
     // (set-up and zsme_set_launch only).
     int ensure_tiles() {
-        if (lc_.tile_faces <= 0 || tile_built_ == lc_.tile_faces) return ZSME_OK;
+        if (lc_.tile_faces <= 0 || (tile_built_ == lc_.tile_faces && (st_built_ == lc_.tile_faces || !wants_stage())))
+            return ZSME_OK;
         FaceTiles t;
         int rc = build_tiles(pm_, lc_.tile_faces, t);
         if (rc) return rc;
+        if (wants_stage() && (rc = upload_stage_tiles(t))) return rc;
+        if (tile_built_ == lc_.tile_faces) return ZSME_OK;
         ZSME_CUDA(tile_cell_off_.upload(t.cell_off, stream_));
         ZSME_CUDA(tile_face_off_.upload(t.face_off, stream_));
         ZSME_CUDA(tile_in_off_.upload(t.in_off, stream_));
@@ -252,7 +263,8 @@ class Solver final : public SolverBase {
         ZSME_CUDA(tile_ord_lf_.upload(t.ord_lf, stream_));
         tile_n_ = t.n;
         tile_stride_ = t.max_faces;
-        const int smem = (int)((size_t)tile_stride_ * 3 * NQ * sizeof(double));
+        // a limit of the kernel, shared by every handle: always the largest
+        const int smem = (int)kMaxTileSmem;
         ZSME_CUDA(cudaFuncSetAttribute(flux_tile_kernel<M, N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         ZSME_CUDA(cudaFuncSetAttribute(flux_tile_kernel<M, N, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         ZSME_CUDA(cudaFuncSetAttribute(flux_tile_kernel<M, N, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -261,6 +273,127 @@ class Solver final : public SolverBase {
         return ZSME_OK;
     }
     LaunchConfig launch() const override { return lc_; }
+
+    // The launch a handle starts with.  With the whole-stage kernel: the
+    // smallest tiles (of at least 96 faces) that still fill the chip in one
+    // wave, because within one wave a step's time is a tile's latency, and then
+    // several threads per cell where a tile's cells leave threads of the block
+    // idle; where one wave of the largest tiles does not cover the mesh, 256
+    // faces, the least rim per cell that leaves kStageBlocks blocks room in
+    // shared memory.  us per step on a B200, level 4 at 15.8 k cells: 96 faces
+    // and 2 threads per cell 45.1, 256 and 1 56.5; level 2 at 51.2 k cells: 320
+    // faces 61.6, 256 71.5, 128 66.1; level 4 at 231 k cells: 256 342, 128 354,
+    // 64 408.  Without it (positivity variants): face + gather tiles of
+    // up to 256 faces, smaller while the mesh would give fewer than three tiles
+    // per SM.
+    void default_tiles(LaunchConfig& lc) const {
+        int tf = std::min(256, (int)(kMaxTileSmem / (3 * NQ * sizeof(double))));
+        if (st_.positivity != ZSME_POSITIVITY_NONE) {
+            while (tf > 64 && pm_.F / tf < 3 * sm_count_) tf /= 2;
+            lc.tile_faces = tf;
+            return;
+        }
+        lc.fuse_final = 1;
+        // a tile evaluates about 1 / 0.87 of the faces it owns; its rows take
+        // about 1.06 cells and 3 NQ doubles per face
+        const int room = (int)((kMaxStageSmem / kStageBlocks - 2048) / (8 * (1.06 * (NQ + 4) + 3 * NQ)));
+        const int largest = std::min(320, room / 32 * 32);
+        const int wave = (int)(pm_.F / (0.87 * kStageBlocks * sm_count_));
+        const int one = std::max(96, (wave + 31) / 32 * 32);
+        lc.tile_faces = one <= largest ? one : std::min(tf, largest);
+        const int entries = (int)(0.85 * lc.tile_faces);   // cells with ring 1, triangles
+        lc.prep_lean = one > largest || 2 * entries > kStageThreads ? 1 : (4 * entries > kStageThreads ? 2 : 4);
+    }
+
+    // ------------------------------------------------------- whole-stage kernel
+    static constexpr int kStageThreads = 256;
+    static constexpr size_t kMaxStageSmem = 227 * 1024;
+        // blocks per SM, which caps the registers: 128 per thread, 80 where the flux
+    // needs no more (level 0: 380 against 436 us per step at 977 k cells; level 2
+    // with 80: 468 against 414 at 498 k cells, spilling)
+    static constexpr int kStageBlocks = NQ >= 6 ? 2 : 3;
+    bool wants_stage() const {
+        return lc_.tile_faces > 0 && lc_.fuse_final && st_.positivity == ZSME_POSITIVITY_NONE;
+    }
+    // the stage kernel serves the step's stages and right-hand sides
+    bool use_stage() const { return wants_stage() && st_built_ == lc_.tile_faces && st_fits_; }
+    int stage_parts() const { return lc_.prep_lean >= 3 ? 4 : (lc_.prep_lean == 2 ? 2 : 1); }
+    int upload_stage_tiles(const FaceTiles& t) {
+        StageTiles s;
+        int rc = build_stage_tiles(pm_, t, st_.reconstruction_order, st_.gradient != ZSME_GRADIENT_LSQ, s);
+        if (rc) return rc;
+        st_built_ = lc_.tile_faces;
+        st_fst_ = t.max_faces + 1;
+        st_cst_ = s.max_local;
+        size_t smem = 0;
+        for (int p : {1, 2, 4}) smem = std::max(smem, stage_smem(p));
+        st_fits_ = s.fits && smem <= kMaxStageSmem;
+        if (!st_fits_) return ZSME_OK;   // the separate stage kernels run instead
+        auto up = [&](DevBuf<int>& d, std::vector<int>& v) {
+            if (v.empty()) v.push_back(0);
+            return d.upload(v, stream_);
+        };
+        std::vector<StageTile> tiles(t.n);
+        for (int b = 0; b < t.n; ++b) {
+            StageTile& d = tiles[b];
+            d.c0 = t.cell_off[b];
+            d.n = t.cell_off[b + 1] - d.c0;
+            d.e0 = s.ext_off[b];
+            d.nloc = d.n + s.ext_off[b + 1] - d.e0;
+            d.nent = d.n + s.ring1[b];
+            d.eo = s.ent_off[b];
+            d.f0 = t.face_off[b];
+            d.nown = t.face_off[b + 1] - d.f0;
+            d.in0 = t.in_off[b];
+            d.nf = d.nown + t.in_off[b + 1] - d.in0;
+            d.g0 = s.gho_off[b];
+            d.ng = s.gho_off[b + 1] - d.g0;
+        }
+        ZSME_CUDA(st_tile_.upload(tiles, stream_));
+        ZSME_CUDA(up(st_ext_cell_, s.ext_cell));
+        ZSME_CUDA(up(st_gho_cell_, s.gho_cell));
+        ZSME_CUDA(up(st_gho_face_, s.gho_face));
+        ZSME_CUDA(st_loc_.upload(s.loc, stream_));
+        st_entries_ = s.ent_off.back();
+        ZSME_CUDA(st_geo_.alloc((size_t)(2 * pm_.K * DIM + 2) * st_entries_));
+        stage_entries_kernel<<<t.n, 128, 0, stream_>>>(md_, st_tile_.p, st_ext_cell_.p, st_loc_.p, st_entries_, DIM,
+                                                       st_.gradient == ZSME_GRADIENT_LSQ, st_geo_.p);
+        ZSME_CUDA(cudaGetLastError());
+        const int bytes = (int)kMaxStageSmem;   // a limit of the kernel, shared by every handle
+#define ZSME_STAGE_ATTR(P)                                                                                            ZSME_CUDA(cudaFuncSetAttribute(stage_kernel<M, N, P, 3, kStageThreads, kStageBlocks>,                                                            cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));                              ZSME_CUDA(cudaFuncSetAttribute(stage_kernel<M, N, P, 4, kStageThreads, kStageBlocks>,                                                            cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        ZSME_STAGE_ATTR(1) ZSME_STAGE_ATTR(2) ZSME_STAGE_ATTR(4)
+#undef ZSME_STAGE_ATTR
+        return ZSME_OK;
+    }
+    int stage_row(int parts, int n) const {
+        return parts == 4 ? StageShape<NQ, 4>::row(n) : (parts == 2 ? StageShape<NQ, 2>::row(n) : StageShape<NQ, 1>::row(n));
+    }
+    size_t stage_smem(int parts) const {
+        return stage_smem_doubles<NQ>(stage_row(parts, st_fst_), stage_row(parts, st_cst_)) * sizeof(double);
+    }
+    // One stage (or right-hand side) of the state x_in; x_out is another buffer.
+    void launch_stage(int mode, double t_host, const double* t_dev, double frac, const double* x_in, double* x_out,
+                      double* base, const double* dt, const int* active) {
+        mark(ZSME_KERNEL_FLUX, true);
+        const int P = stage_parts(), fst = stage_row(P, st_fst_), cst = stage_row(P, st_cst_);
+        const StageTilesDev tl{st_tile_.p, tile_in_faces_.p, tile_ord_lf_.p, st_ext_cell_.p, st_gho_cell_.p,
+                               st_gho_face_.p, st_loc_.p, st_geo_.p, st_entries_, fst, cst};
+        const int s = opts_.stages;
+        const StageWeights sc{(s - 1.) / s, 1. / s, mode == MODE_EULER ? 1.0 : (mode == MODE_FINAL ? s : s - 1.)};
+        const int threads = std::min(kStageThreads, P > 1 ? kStageThreads : (st_fst_ + 31) / 32 * 32);
+#define ZSME_STAGE(PP, KK)                                                                                            stage_kernel<M, N, PP, KK, kStageThreads, kStageBlocks><<<tile_n_, threads, stage_smem(P), stream_>>>(                 md_, opts_, tl, sc, x_in, aux_.p, params_.p, t_host, t_dev, frac, dt, active, mode, x_out, base)
+        if (pm_.K == 3) {
+            if (P == 4) ZSME_STAGE(4, 3);
+            else if (P == 2) ZSME_STAGE(2, 3);
+            else ZSME_STAGE(1, 3);
+        } else {
+            if (P == 4) ZSME_STAGE(4, 4);
+            else if (P == 2) ZSME_STAGE(2, 4);
+            else ZSME_STAGE(1, 4);
+        }
+#undef ZSME_STAGE
+        mark(ZSME_KERNEL_FLUX, false);
+    }
 
     int init(PreparedMesh&& pm, const zsme_settings& st, const double* params, int device) override {
         pm_ = std::move(pm);
@@ -287,11 +420,7 @@ class Solver final : public SolverBase {
         ZSME_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
         ZSME_CUDA(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device_));
         LaunchConfig lc{128, 128, 128, 128};
-        // fused face + gather tiles of up to 256 faces, smaller while the mesh
-        // would give fewer than three tiles per SM
-        int tf = std::min(256, (int)(kMaxTileSmem / (3 * NQ * sizeof(double))));
-        while (tf > 64 && pm_.F / tf < 3 * sm_count_) tf /= 2;
-        lc.tile_faces = tf;
+        default_tiles(lc);
         if (st_.block_size > 0) lc.prep = lc.face = lc.gather = st_.block_size;
         int rc = set_launch(lc);
         if (rc) return rc;
@@ -754,8 +883,10 @@ class Solver final : public SolverBase {
         mark(ZSME_KERNEL_GATHER, false);
     }
     // fg: the last SSP stage's gather, fused into the finalize kernel (or nullptr)
+    // x_src: the state to finalize where it is not x_ itself (the last stage's output buffer)
     void finalize_range(int c0, int cn, const StepDev& sd, const double* dt_src, int flags,
-                        const FinalGather* fg = nullptr) {
+                        const FinalGather* fg = nullptr, const double* x_src = nullptr) {
+        if (!x_src) x_src = x_.p;
         const int gb = blocks_for(cn, lc_.finalize);
         if (flags & FIN_SOURCE) cudaMemsetAsync(sd.n_fallback, 0, sizeof(int), stream_);
         mark(ZSME_KERNEL_FINALIZE, true);
@@ -763,7 +894,7 @@ class Solver final : public SolverBase {
             switch (lc_.finalize_occ) {
 #define ZSME_FING(OCC)                                                                                           \
     case OCC:                                                                                                    \
-        finalize_kernel<M, N, OCC, true><<<gb, lc_.finalize, 0, stream_>>>(md_, c0, cn, x_.p, aux_.p, params_.p,  \
+        finalize_kernel<M, N, OCC, true><<<gb, lc_.finalize, 0, stream_>>>(md_, c0, cn, x_src, x_.p, aux_.p, params_.p,  \
                                                                            sd, dt_src, flags, *fg);              \
         break;
                 ZSME_FING(2) ZSME_FING(3) ZSME_FING(4)
@@ -774,7 +905,7 @@ class Solver final : public SolverBase {
             switch (lc_.finalize_occ) {
 #define ZSME_FIN(OCC)                                                                                            \
     case OCC:                                                                                                    \
-        finalize_kernel<M, N, OCC><<<gb, lc_.finalize, 0, stream_>>>(md_, c0, cn, x_.p, aux_.p, params_.p, sd,    \
+        finalize_kernel<M, N, OCC><<<gb, lc_.finalize, 0, stream_>>>(md_, c0, cn, x_src, x_.p, aux_.p, params_.p, sd,    \
                                                                      dt_src, flags);                             \
         break;
                 ZSME_FIN(2) ZSME_FIN(3) ZSME_FIN(4)
@@ -786,12 +917,27 @@ class Solver final : public SolverBase {
         if (flags & FIN_SOURCE) {   // the cells whose Newton update needs the generic GEPP (usually none)
             mark(ZSME_KERNEL_FALLBACK, true);
             finalize_fallback_kernel<M, N><<<std::min(blocks_for(cn, 64), 8 * sm_count_), 64, 0, stream_>>>(
-                md_, x_.p, aux_.p, params_.p, sd, dt_src, flags);
+                md_, x_src, x_.p, aux_.p, params_.p, sd, dt_src, flags);
             mark(ZSME_KERNEL_FALLBACK, false);
         }
     }
-    void launch_finalize(const StepDev& sd, const double* dt_src, int flags, const FinalGather* fg = nullptr) {
-        finalize_range(0, pm_.C, sd, dt_src, flags, fg);
+    void launch_finalize(const StepDev& sd, const double* dt_src, int flags, const FinalGather* fg = nullptr,
+                         const double* x_src = nullptr) {
+        finalize_range(0, pm_.C, sd, dt_src, flags, fg, x_src);
+    }
+    // FormRHS of the state w into out; w_clamped: its clamped copy, nullptr to form it in wl_
+    void launch_rhs(const double* w, const double* w_clamped, double t_host, const double* t_dev, double frac,
+                    double* out, const double* dt, const int* act) {
+        if (use_stage()) {
+            launch_stage(MODE_RHS, t_host, t_dev, frac, w, out, nullptr, dt, act);
+            return;
+        }
+        if (!w_clamped) {
+            clamp_kernel<M><<<blocks_for(pm_.C, 128), 128, 0, stream_>>>(md_, 0, pm_.C, w, aux_.p, params_.p, wl_.p);
+            w_clamped = wl_.p;
+        }
+        launch_prep(w, w_clamped, act);
+        launch_flux(MODE_RHS, t_host, t_dev, frac, nullptr, out, nullptr, dt, act);
     }
 
     int rhs(double t, const double* x_aos, double* f_aos) override {
@@ -799,9 +945,7 @@ class Solver final : public SolverBase {
         const int C = pm_.C;
         ZSME_CUDA(cudaMemcpyAsync(tmp_b_.p, x_aos, (size_t)NQ * C * sizeof(double), cudaMemcpyHostToDevice, stream_));
         aos_to_soa_kernel<<<blocks_for(C, 128), 128, 0, stream_>>>(tmp_b_.p, w_.p, old_of_new_.p, 0, C, C, NQ);
-        clamp_kernel<M><<<blocks_for(C, 128), 128, 0, stream_>>>(md_, 0, C, w_.p, aux_.p, params_.p, wl_.p);
-        launch_prep(w_.p, wl_.p, nullptr);
-        launch_flux(MODE_RHS, t, nullptr, 0.0, nullptr, tmp_a_.p, nullptr, nullptr, nullptr);
+        launch_rhs(w_.p, nullptr, t, nullptr, 0.0, tmp_a_.p, nullptr, nullptr);
         ZSME_CUDA(cudaGetLastError());
         return get_soa(0, tmp_a_.p, NQ, f_aos, false);
     }
@@ -875,9 +1019,27 @@ class Solver final : public SolverBase {
         const bool fuse_final = lc_.fuse_final && lc_.tile_faces == 0 && st_.reconstruction_order >= 2 && !mood &&
                                 !tape && !deriv_.n && st_.time_integration == ZSME_TIME_SPLITTING;
         double* w_last = x_.p;   // the last stage's state
+        const double* x_new = x_.p;   // the transport result
+        const bool stage = use_stage() && !tape;
         const bool imex = st_.time_integration == ZSME_TIME_IMEX;
         if (imex) {
             enqueue_imex_stages(t, dt, act, wl0);
+        } else if (stage && st_.reconstruction_order < 2) {
+            launch_derivative_aux(x_.p, act);       // FormRHS's UpdateState of the stage state
+            launch_stage(MODE_EULER, 0.0, t, 0.0, x_.p, w_.p, nullptr, dt, act);
+            x_new = w_.p;   // other tiles read x_ while this one is written
+        } else if (stage) {
+            // a stage's output never is its input: the states alternate between w_ and wl_
+            const int s = st_.ssp_stages;
+            for (int i = 0; i < s; ++i) {
+                launch_derivative_aux(w_last, act);
+                double* w_out = i % 2 == 0 ? w_.p : wl_.p;
+                if (i < s - 1)
+                    launch_stage(i == 0 ? MODE_FIRST : MODE_MID, 0.0, t, i / (s - 1.), w_last, w_out, nullptr, dt, act);
+                else
+                    launch_stage(MODE_FINAL, 0.0, t, 1.0, w_last, nullptr, x_.p, dt, act);
+                w_last = w_out;
+            }
         } else if (st_.reconstruction_order < 2) {
             launch_derivative_aux(x_.p, act);       // FormRHS's UpdateState of the stage state
             stage_fs(0);
@@ -924,8 +1086,8 @@ class Solver final : public SolverBase {
         const FinalGather fg{fb_.p, w_last, sd.dt_step, st_.ssp_stages};
         // EnforcePhysicalConstraints' UpdateState: the derivative aux of the
         // transport result before the constraints and the source
-        launch_derivative_aux(x_.p, act);
-        launch_finalize(sd, sd.dt_step, flags, fuse_final ? &fg : nullptr);
+        launch_derivative_aux(x_new, act);
+        launch_finalize(sd, sd.dt_step, flags, fuse_final ? &fg : nullptr, x_new);
         launch_derivative_aux(x_.p, act);           // PostStep's UpdateState
         mark(ZSME_KERNEL_END, true);
         end_step_kernel<<<blocks_for(n_inst_, 128), 128, 0, stream_>>>(sd, 0, n_inst_, 1, 0.0, nullptr);
@@ -940,22 +1102,19 @@ class Solver final : public SolverBase {
         const int C = pm_.C, nb = blocks_for(C, 128);
         auto rhs = [&](double* y, const double* wl, double frac, double* g) {
             launch_derivative_aux(y, act);
-            launch_prep(y, wl, act);
-            launch_flux(MODE_RHS, 0.0, t, frac, nullptr, g, nullptr, dt, act);
+            launch_rhs(y, wl, 0.0, t, frac, g, dt, act);
         };
         rhs(x_.p, wl0, 0.0, imex_g_[0].p);
         imex_source_kernel<M><<<nb, 128, 0, stream_>>>(md_, x_.p, aux_.p, params_.p, imex_s_[0].p, act);
         const ImexTerms t1{{imex_g_[0].p}, {imex_s_[0].p}, {K::a10}, {K::t10}, 1};
         imex_stage_kernel<M><<<blocks_for(C, 64), 64, 0, stream_>>>(md_, t1, x_.p, aux_.p, params_.p, dt, act,
                                                                     imex_y_[0].p, imex_s_[1].p, iscal_.p + 1);
-        clamp_kernel<M><<<nb, 128, 0, stream_>>>(md_, 0, C, imex_y_[0].p, aux_.p, params_.p, wl_.p);
-        rhs(imex_y_[0].p, wl_.p, K::c1, imex_g_[1].p);
+        rhs(imex_y_[0].p, nullptr, K::c1, imex_g_[1].p);
         const ImexTerms t2{{imex_g_[0].p, imex_g_[1].p}, {imex_s_[0].p, imex_s_[1].p}, {K::a20, K::a21},
                            {K::t20, K::t21}, 2};
         imex_stage_kernel<M><<<blocks_for(C, 64), 64, 0, stream_>>>(md_, t2, x_.p, aux_.p, params_.p, dt, act,
                                                                     imex_y_[1].p, imex_s_[2].p, iscal_.p + 1);
-        clamp_kernel<M><<<nb, 128, 0, stream_>>>(md_, 0, C, imex_y_[1].p, aux_.p, params_.p, wl_.p);
-        rhs(imex_y_[1].p, wl_.p, K::c2, imex_g_[2].p);
+        rhs(imex_y_[1].p, nullptr, K::c2, imex_g_[2].p);
         const ImexTerms tb{{imex_g_[0].p, imex_g_[1].p, imex_g_[2].p},
                            {imex_s_[0].p, imex_s_[1].p, imex_s_[2].p},
                            {K::b0, K::b1, K::b2},
@@ -996,9 +1155,7 @@ class Solver final : public SolverBase {
     // the time in device memory (the step's), else t
     void imp_residual(double t, const double* y, const BdfTerms& b, double* f, const double* t_dev = nullptr) {
         const int C = pm_.C;
-        clamp_kernel<M><<<blocks_for(C, 128), 128, 0, stream_>>>(md_, 0, C, y, aux_.p, params_.p, wl_.p);
-        launch_prep(y, wl_.p, nullptr);
-        launch_flux(MODE_RHS, t, t_dev, 0.0, nullptr, imp_R_.p, nullptr, nullptr, nullptr);
+        launch_rhs(y, nullptr, t, t_dev, 0.0, imp_R_.p, nullptr, nullptr);
         imp_residual_kernel<M><<<blocks_for(C, 128), 128, 0, stream_>>>(md_, y, aux_.p, params_.p, imp_R_.p, b, f);
     }
     // the step's residual: time and BDF coefficients from imp_scal_
@@ -1307,10 +1464,10 @@ class Solver final : public SolverBase {
     }
     int launches_per_step() const override {
         if (st_.time_integration == ZSME_TIME_IMEX) {
-            const int per_rhs = (lc_.tile_faces > 0 ? 2 : 3) + (deriv_.n ? 1 : 0);
-            return 3 + 3 * per_rhs + 6 + (deriv_.n ? 2 : 0) + (st_.positivity == ZSME_POSITIVITY_MOOD ? 2 : 0);
+            const int per_rhs = (use_stage() ? 1 : (lc_.tile_faces > 0 ? 2 : 3)) + (deriv_.n ? 1 : 0);
+            return 3 + 3 * per_rhs + (use_stage() ? 4 : 6) + (deriv_.n ? 2 : 0) + (st_.positivity == ZSME_POSITIVITY_MOOD ? 2 : 0);
         }
-        const int per_stage = lc_.tile_faces > 0 ? 2 : 3;
+        const int per_stage = use_stage() ? 1 : (lc_.tile_faces > 0 ? 2 : 3);
         const bool fuse_final = lc_.fuse_final && lc_.tile_faces == 0 && st_.reconstruction_order >= 2 &&
                                 st_.positivity != ZSME_POSITIVITY_MOOD && !deriv_.n;
         const int derivs = deriv_.n ? (st_.reconstruction_order < 2 ? 1 : st_.ssp_stages) + 2 : 0;

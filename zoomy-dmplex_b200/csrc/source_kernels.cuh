@@ -204,9 +204,10 @@ enum FinalizeFlags {
 // CFL ratio (into ratio).  GENERIC = false: returns -1 without storing
 // anything when the Newton iteration needs the generic full-size GEPP.
 // GATHER: the cell's state is the last SSP stage's result, formed here from
-// the face contributions (gather_final_state) instead of read from x.
+// the face contributions (gather_final_state) instead of read from x_src (x
+// itself, or the last stage's output buffer).
 template <class M, class N, bool GENERIC, bool GATHER = false>
-__device__ __forceinline__ int finalize_cell(const MeshDev& m, int c, int I, double* __restrict__ x,
+__device__ __forceinline__ int finalize_cell(const MeshDev& m, int c, int I, const double* x_src, double* x,
                                              double* __restrict__ aux, const double* p, const StepDev& sd,
                                              const double* __restrict__ dt_src, int flags, double& ratio,
                                              const FinalGather* fg = nullptr) {
@@ -214,7 +215,7 @@ __device__ __forceinline__ int finalize_cell(const MeshDev& m, int c, int I, dou
     const int C = m.C;
     double q[NQ], a[NA];
     if constexpr (GATHER) gather_final_state<M>(m, c, I, *fg, x, q);
-    else load_q<NQ>(x, C, c, q);
+    else load_q<NQ>(x_src, C, c, q);
 #pragma unroll
     for (int i = 0; i < NA; ++i) a[i] = aux[(size_t)i * C + c];
     if (flags & FIN_PRE) constrain<M>(q, a, p);
@@ -324,9 +325,9 @@ __device__ __forceinline__ void block_ratio_min(const StepDev& sd, int I, double
 // stage result never round-trips through x; a deferred cell gets that result
 // written to x for finalize_fallback_kernel.
 template <class M, class N, int MINB, bool GATHER = false>
-__global__ void __launch_bounds__(128, MINB) finalize_kernel(MeshDev m, int c0, int cn, double* __restrict__ x,
-                                                       double* __restrict__ aux, const double* __restrict__ params,
-                                                       StepDev sd, const double* __restrict__ dt_src, int flags,
+__global__ void __launch_bounds__(128, MINB) finalize_kernel(MeshDev m, int c0, int cn, const double* x_src,
+                                                       double* x, double* __restrict__ aux,
+                                                       const double* __restrict__ params, StepDev sd, const double* __restrict__ dt_src, int flags,
                                                        FinalGather fg = FinalGather{}) {
     constexpr int NQ = M::n_dof_q;
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -335,7 +336,7 @@ __global__ void __launch_bounds__(128, MINB) finalize_kernel(MeshDev m, int c0, 
     double ratio = DBL_MAX;
     const bool act = I >= 0 && (sd.active ? (sd.active[I] != 0) : true);
     bool defer = false;
-    if (act) defer = finalize_cell<M, N, false, GATHER>(m, c, I, x, aux, params + (size_t)I * m.np, sd, dt_src,
+    if (act) defer = finalize_cell<M, N, false, GATHER>(m, c, I, x_src, x, aux, params + (size_t)I * m.np, sd, dt_src,
                                                          flags, ratio, &fg) < 0;
     if constexpr (GATHER) {
         if (defer) {   // the generic path restarts from the stage result
@@ -353,7 +354,7 @@ __global__ void __launch_bounds__(128, MINB) finalize_kernel(MeshDev m, int c0, 
 // (grid-stride over sd.fallback[0 .. *sd.n_fallback)); their CFL ratios go
 // straight to the per-instance atomic minimum, which is order-free.
 template <class M, class N>
-__global__ void __launch_bounds__(64) finalize_fallback_kernel(MeshDev m, double* __restrict__ x,
+__global__ void __launch_bounds__(64) finalize_fallback_kernel(MeshDev m, const double* x_src, double* x,
                                                                double* __restrict__ aux,
                                                                const double* __restrict__ params, StepDev sd,
                                                                const double* __restrict__ dt_src, int flags) {
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(64) finalize_fallback_kernel(MeshDev m, double
         const int c = sd.fallback[e];
         const int I = cell_instance(m, c);
         double ratio = DBL_MAX;
-        finalize_cell<M, N, true>(m, c, I, x, aux, params + (size_t)I * m.np, sd, dt_src, flags, ratio);
+        finalize_cell<M, N, true>(m, c, I, x_src, x, aux, params + (size_t)I * m.np, sd, dt_src, flags, ratio);
         if ((flags & FIN_DT) && ratio < DBL_MAX)
             atomicMin(&sd.ratio[I], (unsigned long long)__double_as_longlong(ratio));
     }

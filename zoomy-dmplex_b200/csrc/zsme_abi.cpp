@@ -124,7 +124,7 @@ int zsme_create(const char* model, const zsme_mesh* mesh, const zsme_settings* s
     if (settings->positivity < ZSME_POSITIVITY_NONE || settings->positivity > ZSME_POSITIVITY_MOOD)
         return set_error(ZSME_ERR_ARG, "positivity must be ZSME_POSITIVITY_NONE, _ZHANG_SHU or _MOOD");
     zsme::PreparedMesh pm;
-    int rc = zsme::prepare_mesh(*mesh, pm);
+    int rc = zsme::prepare_mesh(*mesh, pm, settings->gradient == ZSME_GRADIENT_LSQ);
     if (rc) return rc;
     DeviceGuard dev_guard(device);
     if ((rc = dev_guard.check())) return rc;
@@ -337,7 +337,7 @@ int zsme_batch_create(const char* model, int32_t n, const zsme_mesh* meshes, con
         return set_error(ZSME_ERR_ARG, "positivity must be ZSME_POSITIVITY_NONE, _ZHANG_SHU or _MOOD");
     std::vector<zsme::PreparedMesh> parts(n);
     for (int i = 0; i < n; ++i) {
-        int rc = zsme::prepare_mesh(meshes[i], parts[i]);
+        int rc = zsme::prepare_mesh(meshes[i], parts[i], settings->gradient == ZSME_GRADIENT_LSQ);
         if (rc) return set_error(rc, "instance " + std::to_string(i) + ": " + zsme_last_error());
     }
     zsme::PreparedMesh pm;

@@ -373,10 +373,12 @@ LAUNCH_DEFAULTS = {"prep": 128, "face": 128, "gather": 128, "finalize": 128, "pr
 def set_launch(h, cfg):
     """Launch configuration of a handle: dict with LAUNCH_KEYS (threads per
     block of each kernel, register caps as blocks per SM, tile_faces: 0 for
-    the separate face and gather kernels, else the fused tile kernel's most
-    faces per tile, fuse_final: the last stage's gather inside the finalize
-    kernel, prep_lean: the lean face-state kernel); missing keys take
-    LAUNCH_DEFAULTS."""
+    the separate face and gather kernels, else the tile kernels' most faces
+    per tile, fuse_final: with tiles the whole stage in one kernel, else the
+    last stage's gather inside the finalize kernel, prep_lean: the lean
+    face-state kernel and its threads per cell); missing keys take
+    LAUNCH_DEFAULTS.  A new handle has the configuration that get_launch
+    returns, chosen by model and mesh size."""
     lib = native.load()
     b = (ct.c_int32 * len(LAUNCH_KEYS))(*[int(cfg.get(k, LAUNCH_DEFAULTS[k])) for k in LAUNCH_KEYS])
     native.check(lib.zsme_set_launch(h, b))
