@@ -102,8 +102,9 @@ class Solver final : public SolverBase {
     int imp_stats_[4] = {0, 0, 0, 0};   // last step: Newton iterations, GMRES iterations, halvings, converged
 
     // per instance: t, dt_cfl, dt_step, dt_aux ; active ; ratio
-    DevBuf<double> t_, dt_cfl_, dt_step_, dt_aux_;
-    DevBuf<int> active_, iscal_;  // iscal_: [0] step_idx, [1..4] diag, [5] deferred finalize cells, [6] MOOD cells
+    DevBuf<double> t_, dt_cfl_, dt_step_, dt_aux_, dt_last_;
+    DevBuf<int> active_, iscal_;  // iscal_: [0] step_idx, [1..4] diag, [5] deferred finalize cells, [6] MOOD cells,
+                                  // [7] diag's deferred cells, [8] blocks done in step_tail_kernel
     DevBuf<int> fin_list_;        // [C] cells deferred to the generic Newton path
     // tiles of the fused face + gather kernel (LaunchConfig::tile_faces > 0)
     DevBuf<int> tile_cell_off_, tile_face_off_, tile_in_off_, tile_in_faces_, tile_ord_lf_;
@@ -305,6 +306,23 @@ class Solver final : public SolverBase {
         lc.prep_lean = one > largest || 2 * entries > kStageThreads ? 1 : (4 * entries > kStageThreads ? 2 : 4);
     }
 
+    // A launch that may start while its predecessor drains (grid_wait in the
+    // kernel); per-kernel timing keeps the kernels apart.
+    template <class... KA, class... A>
+    void launch_chained(void (*k)(KA...), int grid, int block, size_t smem, A... args) {
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(block);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream_;
+        cfg.attrs = &attr;
+        cfg.numAttrs = profiling_ ? 0 : 1;
+        cudaLaunchKernelEx(&cfg, k, KA(args)...);
+    }
+
     // ------------------------------------------------------- whole-stage kernel
     static constexpr int kStageThreads = 256;
     static constexpr size_t kMaxStageSmem = 227 * 1024;
@@ -359,6 +377,7 @@ class Solver final : public SolverBase {
         stage_entries_kernel<<<t.n, 128, 0, stream_>>>(md_, st_tile_.p, st_ext_cell_.p, st_loc_.p, st_entries_, DIM,
                                                        st_.gradient == ZSME_GRADIENT_LSQ, st_geo_.p);
         ZSME_CUDA(cudaGetLastError());
+        ZSME_CUDA(cudaStreamSynchronize(stream_));   // a chained launch reads it without waiting for the stream
         const int bytes = (int)kMaxStageSmem;   // a limit of the kernel, shared by every handle
 #define ZSME_STAGE_ATTR(P)                                                                                            ZSME_CUDA(cudaFuncSetAttribute(stage_kernel<M, N, P, 3, kStageThreads, kStageBlocks>,                                                            cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));                              ZSME_CUDA(cudaFuncSetAttribute(stage_kernel<M, N, P, 4, kStageThreads, kStageBlocks>,                                                            cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
         ZSME_STAGE_ATTR(1) ZSME_STAGE_ATTR(2) ZSME_STAGE_ATTR(4)
@@ -381,7 +400,9 @@ class Solver final : public SolverBase {
         const int s = opts_.stages;
         const StageWeights sc{(s - 1.) / s, 1. / s, mode == MODE_EULER ? 1.0 : (mode == MODE_FINAL ? s : s - 1.)};
         const int threads = std::min(kStageThreads, P > 1 ? kStageThreads : (st_fst_ + 31) / 32 * 32);
-#define ZSME_STAGE(PP, KK)                                                                                            stage_kernel<M, N, PP, KK, kStageThreads, kStageBlocks><<<tile_n_, threads, stage_smem(P), stream_>>>(                 md_, opts_, tl, sc, x_in, aux_.p, params_.p, t_host, t_dev, frac, dt, active, mode, x_out, base)
+#define ZSME_STAGE(PP, KK)                                                                                        \
+    launch_chained(stage_kernel<M, N, PP, KK, kStageThreads, kStageBlocks>, tile_n_, threads, stage_smem(P), md_,  \
+                   opts_, tl, sc, x_in, aux_.p, params_.p, t_host, t_dev, frac, dt, active, mode, x_out, base)
         if (pm_.K == 3) {
             if (P == 4) ZSME_STAGE(4, 3);
             else if (P == 2) ZSME_STAGE(2, 3);
@@ -488,15 +509,15 @@ class Solver final : public SolverBase {
         ZSME_CUDA(tmp_b_.alloc((size_t)std::max(NQ, NA) * C));
         ZSME_CUDA(cudaMemsetAsync(x_.p, 0, x_.n * sizeof(double), stream_));
         ZSME_CUDA(cudaMemsetAsync(aux_.p, 0, aux_.n * sizeof(double), stream_));
-        for (auto* b : {&t_, &dt_cfl_, &dt_step_, &dt_aux_}) {
+        for (auto* b : {&t_, &dt_cfl_, &dt_step_, &dt_aux_, &dt_last_}) {
             ZSME_CUDA(b->alloc(n_inst_));
             ZSME_CUDA(cudaMemsetAsync(b->p, 0, n_inst_ * sizeof(double), stream_));
         }
         ZSME_CUDA(fin_list_.alloc((size_t)C));
         ZSME_CUDA(active_.alloc(n_inst_));
         ZSME_CUDA(cudaMemsetAsync(active_.p, 0, n_inst_ * sizeof(int), stream_));
-        ZSME_CUDA(iscal_.alloc(8));
-        ZSME_CUDA(cudaMemsetAsync(iscal_.p, 0, 8 * sizeof(int), stream_));
+        ZSME_CUDA(iscal_.alloc(16));
+        ZSME_CUDA(cudaMemsetAsync(iscal_.p, 0, 16 * sizeof(int), stream_));
         ZSME_CUDA(ratio_.alloc(n_inst_));
         std::vector<unsigned long long> none(n_inst_, ZSME_RATIO_NONE);
         ZSME_CUDA(cudaMemcpyAsync(ratio_.p, none.data(), n_inst_ * sizeof(unsigned long long),
@@ -568,7 +589,8 @@ class Solver final : public SolverBase {
 
     StepDev step_dev(const double* dts) {
         return StepDev{t_.p, dt_cfl_.p, dt_step_.p, active_.p, ratio_.p, dts, iscal_.p + 0, n_inst_,
-                       st_.t_end, st_.cfl, M::dt_max, iscal_.p + 1, fin_list_.p, iscal_.p + 5};
+                       st_.t_end, st_.cfl, M::dt_max, iscal_.p + 1, fin_list_.p, iscal_.p + 5, dt_last_.p,
+                       iscal_.p + 8};
     }
 
     int set_params(const double* params) override {
@@ -883,12 +905,13 @@ class Solver final : public SolverBase {
         mark(ZSME_KERNEL_GATHER, false);
     }
     // fg: the last SSP stage's gather, fused into the finalize kernel (or nullptr)
-    // x_src: the state to finalize where it is not x_ itself (the last stage's output buffer)
+    // x_src: the state to finalize where it is not x_ itself (the last stage's output buffer);
+    // chained: the step's tail with it (step_tail_kernel), sd.n_fallback being zero
     void finalize_range(int c0, int cn, const StepDev& sd, const double* dt_src, int flags,
-                        const FinalGather* fg = nullptr, const double* x_src = nullptr) {
+                        const FinalGather* fg = nullptr, const double* x_src = nullptr, bool chained = false) {
         if (!x_src) x_src = x_.p;
         const int gb = blocks_for(cn, lc_.finalize);
-        if (flags & FIN_SOURCE) cudaMemsetAsync(sd.n_fallback, 0, sizeof(int), stream_);
+        if ((flags & FIN_SOURCE) && !chained) cudaMemsetAsync(sd.n_fallback, 0, sizeof(int), stream_);
         mark(ZSME_KERNEL_FINALIZE, true);
         if (fg) {
             switch (lc_.finalize_occ) {
@@ -905,8 +928,8 @@ class Solver final : public SolverBase {
             switch (lc_.finalize_occ) {
 #define ZSME_FIN(OCC)                                                                                            \
     case OCC:                                                                                                    \
-        finalize_kernel<M, N, OCC><<<gb, lc_.finalize, 0, stream_>>>(md_, c0, cn, x_src, x_.p, aux_.p, params_.p, sd,    \
-                                                                     dt_src, flags);                             \
+        launch_chained(finalize_kernel<M, N, OCC>, gb, lc_.finalize, 0, md_, c0, cn, x_src, x_.p, aux_.p,         \
+                       params_.p, sd, dt_src, flags, FinalGather{});                                             \
         break;
                 ZSME_FIN(2) ZSME_FIN(3) ZSME_FIN(4)
                 default: ZSME_FIN(1)
@@ -914,6 +937,11 @@ class Solver final : public SolverBase {
             }
         }
         mark(ZSME_KERNEL_FINALIZE, false);
+        if (chained) {
+            launch_chained(step_tail_kernel<M, N>, std::min(blocks_for(cn, 64), 4 * sm_count_), 64, 0, md_, x_src, x_.p,
+                           aux_.p, params_.p, sd, dt_src, flags);
+            return;
+        }
         if (flags & FIN_SOURCE) {   // the cells whose Newton update needs the generic GEPP (usually none)
             mark(ZSME_KERNEL_FALLBACK, true);
             finalize_fallback_kernel<M, N><<<std::min(blocks_for(cn, 64), 8 * sm_count_), 64, 0, stream_>>>(
@@ -922,8 +950,8 @@ class Solver final : public SolverBase {
         }
     }
     void launch_finalize(const StepDev& sd, const double* dt_src, int flags, const FinalGather* fg = nullptr,
-                         const double* x_src = nullptr) {
-        finalize_range(0, pm_.C, sd, dt_src, flags, fg, x_src);
+                         const double* x_src = nullptr, bool chained = false) {
+        finalize_range(0, pm_.C, sd, dt_src, flags, fg, x_src, chained);
     }
     // FormRHS of the state w into out; w_clamped: its clamped copy, nullptr to form it in wl_
     void launch_rhs(const double* w, const double* w_clamped, double t_host, const double* t_dev, double frac,
@@ -991,7 +1019,9 @@ class Solver final : public SolverBase {
     // tape (adjoint replay): NQ x C slots receiving each stage state W_1 .. W_{s-1}
     // and the stage output X' before finalize (tape[0] = W_0 is the caller's copy),
     // then 2 NQ x F slots receiving each stage's face states
-    void enqueue_step(const double* dts, const double* wl0, double* tape = nullptr) {
+    // chained: the captured form, whose tail kernel also begins the next step; the
+    // first of a run of them follows a begin_steps_kernel
+    void enqueue_step(const double* dts, const double* wl0, double* tape = nullptr, bool chained = false) {
         const size_t tape_n = (size_t)NQ * pm_.C;
         const size_t fs_n = (size_t)2 * NQ * pm_.F;
         const int ns = st_.reconstruction_order < 2 ? 1 : st_.ssp_stages;
@@ -1008,9 +1038,11 @@ class Solver final : public SolverBase {
         const double* t = sd.t;
         const double* dt = sd.dt_step;
         const int* act = sd.active;
-        mark(ZSME_KERNEL_BEGIN, true);
-        begin_step_kernel<<<blocks_for(n_inst_, 128), 128, 0, stream_>>>(sd, 0, n_inst_);
-        mark(ZSME_KERNEL_BEGIN, false);
+        if (!chained) {
+            mark(ZSME_KERNEL_BEGIN, true);
+            begin_step_kernel<<<blocks_for(n_inst_, 128), 128, 0, stream_>>>(sd, 0, n_inst_);
+            mark(ZSME_KERNEL_BEGIN, false);
+        }
         const bool mood = st_.positivity == ZSME_POSITIVITY_MOOD;
         if (mood) cudaMemcpyAsync(xs_.p, x_.p, xs_.n * sizeof(double), cudaMemcpyDeviceToDevice, stream_);
         // the last stage's gather inside finalize: separate face and gather
@@ -1087,8 +1119,11 @@ class Solver final : public SolverBase {
         // EnforcePhysicalConstraints' UpdateState: the derivative aux of the
         // transport result before the constraints and the source
         launch_derivative_aux(x_new, act);
-        launch_finalize(sd, sd.dt_step, flags, fuse_final ? &fg : nullptr, x_new);
-        launch_derivative_aux(x_.p, act);           // PostStep's UpdateState
+        launch_finalize(sd, sd.dt_step, flags, fuse_final ? &fg : nullptr, x_new, chained);
+        // PostStep's UpdateState.  After the tail, active already is the next step's:
+        // every instance is refreshed, which leaves an idle one as it was
+        launch_derivative_aux(x_.p, chained ? nullptr : act);
+        if (chained) return;
         mark(ZSME_KERNEL_END, true);
         end_step_kernel<<<blocks_for(n_inst_, 128), 128, 0, stream_>>>(sd, 0, n_inst_, 1, 0.0, nullptr);
         mark(ZSME_KERNEL_END, false);
@@ -1465,15 +1500,16 @@ class Solver final : public SolverBase {
     int launches_per_step() const override {
         if (st_.time_integration == ZSME_TIME_IMEX) {
             const int per_rhs = (use_stage() ? 1 : (lc_.tile_faces > 0 ? 2 : 3)) + (deriv_.n ? 1 : 0);
-            return 3 + 3 * per_rhs + (use_stage() ? 4 : 6) + (deriv_.n ? 2 : 0) + (st_.positivity == ZSME_POSITIVITY_MOOD ? 2 : 0);
+            return (use_stage() ? 2 : 3) + 3 * per_rhs + (use_stage() ? 4 : 6) + (deriv_.n ? 2 : 0) + (st_.positivity == ZSME_POSITIVITY_MOOD ? 2 : 0);
         }
         const int per_stage = use_stage() ? 1 : (lc_.tile_faces > 0 ? 2 : 3);
         const bool fuse_final = lc_.fuse_final && lc_.tile_faces == 0 && st_.reconstruction_order >= 2 &&
                                 st_.positivity != ZSME_POSITIVITY_MOOD && !deriv_.n;
         const int derivs = deriv_.n ? (st_.reconstruction_order < 2 ? 1 : st_.ssp_stages) + 2 : 0;
-        return 3 + derivs - (fuse_final ? 1 : 0) +
+        // finalize and the step's tail, or begin, finalize, its fallback and the end
+        return (use_stage() ? 2 : 3 + (st_.source ? 1 : 0)) + derivs - (fuse_final ? 1 : 0) +
                (st_.reconstruction_order < 2 ? per_stage : per_stage * st_.ssp_stages) +
-               (st_.positivity == ZSME_POSITIVITY_MOOD ? 2 : 0) + (st_.source ? 1 : 0);
+               (st_.positivity == ZSME_POSITIVITY_MOOD ? 2 : 0);
     }
 
     int step(int nsteps, const double* dts_host) override {
@@ -1484,17 +1520,23 @@ class Solver final : public SolverBase {
             ZSME_CUDA(cudaMemsetAsync(iscal_.p + 7, 0, sizeof(int), stream_));
             return implicit_steps(nsteps, dts_host);
         }
-        ZSME_CUDA(cudaMemsetAsync(iscal_.p + 1, 0, 4 * sizeof(int), stream_));
-        ZSME_CUDA(cudaMemsetAsync(iscal_.p + 7, 0, sizeof(int), stream_));
+        const bool unclamped = !x_clamped_ && st_.reconstruction_order >= 2;
+        const bool plain = dts_host || profiling_ || unclamped;
+        const bool chained = !plain && use_stage();
+        if (chained) {
+            begin_steps_kernel<<<blocks_for(n_inst_, 128), 128, 0, stream_>>>(step_dev(nullptr));
+        } else {
+            ZSME_CUDA(cudaMemsetAsync(iscal_.p + 1, 0, 4 * sizeof(int), stream_));
+            ZSME_CUDA(cudaMemsetAsync(iscal_.p + 7, 0, sizeof(int), stream_));
+        }
         // x_ is constrained after set_state, update_state and every step (update_variables is a
         // projection: the clamp of a clamped state is that state), so it serves as its own
         // clamped copy; after a bare source() the first step clamps a copy first, uncaptured
-        const bool unclamped = !x_clamped_ && st_.reconstruction_order >= 2;
         x_clamped_ = true;
         if (unclamped)
             clamp_kernel<M><<<blocks_for(pm_.C, 128), 128, 0, stream_>>>(md_, 0, pm_.C, x_.p, aux_.p, params_.p,
                                                                         wl_.p);
-        if (dts_host || profiling_ || unclamped) {
+        if (plain) {
             // imposed dts or per-kernel timing: plain launches (the step index
             // lives on the device)
             if (dts_host) {
@@ -1511,7 +1553,7 @@ class Solver final : public SolverBase {
             if (!graph_) {
                 cudaGraph_t g = nullptr;
                 ZSME_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-                enqueue_step(nullptr, x_.p);
+                enqueue_step(nullptr, x_.p, nullptr, chained);
                 ZSME_CUDA(cudaStreamEndCapture(stream_, &g));
                 ZSME_CUDA(cudaGraphInstantiate(&graph_, g, 0));
                 cudaGraphDestroy(g);
@@ -1766,7 +1808,7 @@ class Solver final : public SolverBase {
             obs_values(n);
             int rc = step(1, nullptr);
             if (rc) return rc;
-            ZSME_CUDA(cudaMemcpyAsync(adj_dts_.p + n, dt_step_.p, sizeof(double), cudaMemcpyDeviceToDevice, stream_));
+            ZSME_CUDA(cudaMemcpyAsync(adj_dts_.p + n, dt_last_.p, sizeof(double), cudaMemcpyDeviceToDevice, stream_));
             if ((n + 1) % E == 0 && n + 1 < NS) save((n + 1) / E);
         }
         obs_values(NS);

@@ -330,6 +330,8 @@ __global__ void __launch_bounds__(128, MINB) finalize_kernel(MeshDev m, int c0, 
                                                        const double* __restrict__ params, StepDev sd, const double* __restrict__ dt_src, int flags,
                                                        FinalGather fg = FinalGather{}) {
     constexpr int NQ = M::n_dof_q;
+    grid_release();
+    grid_wait();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     const int c = c0 + r;
     const int I = r < cn ? cell_instance(m, c) : -1;
@@ -351,14 +353,13 @@ __global__ void __launch_bounds__(128, MINB) finalize_kernel(MeshDev m, int c0, 
 }
 
 // The deferred cells of finalize_kernel, with the generic Newton path
-// (grid-stride over sd.fallback[0 .. *sd.n_fallback)); their CFL ratios go
-// straight to the per-instance atomic minimum, which is order-free.
+// (grid-stride over sd.fallback[0 .. n)); their CFL ratios go straight to the
+// per-instance atomic minimum, which is order-free.
 template <class M, class N>
-__global__ void __launch_bounds__(64) finalize_fallback_kernel(MeshDev m, const double* x_src, double* x,
-                                                               double* __restrict__ aux,
-                                                               const double* __restrict__ params, StepDev sd,
-                                                               const double* __restrict__ dt_src, int flags) {
-    const int n = *sd.n_fallback;
+__device__ __forceinline__ void finalize_deferred(const MeshDev& m, const double* x_src, double* x,
+                                                  double* __restrict__ aux, const double* __restrict__ params,
+                                                  const StepDev& sd, const double* __restrict__ dt_src, int flags,
+                                                  int n) {
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(&sd.diag[6], n);
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const int c = sd.fallback[e];
@@ -367,6 +368,48 @@ __global__ void __launch_bounds__(64) finalize_fallback_kernel(MeshDev m, const 
         finalize_cell<M, N, true>(m, c, I, x_src, x, aux, params + (size_t)I * m.np, sd, dt_src, flags, ratio);
         if ((flags & FIN_DT) && ratio < DBL_MAX)
             atomicMin(&sd.ratio[I], (unsigned long long)__double_as_longlong(ratio));
+    }
+}
+template <class M, class N>
+__global__ void __launch_bounds__(64) finalize_fallback_kernel(MeshDev m, const double* x_src, double* x,
+                                                               double* __restrict__ aux,
+                                                               const double* __restrict__ params, StepDev sd,
+                                                               const double* __restrict__ dt_src, int flags) {
+    finalize_deferred<M, N>(m, x_src, x, aux, params, sd, dt_src, flags, *sd.n_fallback);
+}
+
+// The end of a captured step in one launch: finalize_kernel's deferred cells,
+// the step end and the next step's begin (end_step_kernel, begin_step_kernel).
+// Usually no cell is deferred; then block 0 ends the step at once.  Otherwise
+// the last block to finish its cells does.  One launch where a memset, the
+// fallback, the end and the next begin were four (10 of the 42 us of a
+// 1 k-cell level-0 step).
+template <class M, class N>
+__global__ void __launch_bounds__(64) step_tail_kernel(MeshDev m, const double* x_src, double* x,
+                                                       double* __restrict__ aux, const double* __restrict__ params,
+                                                       StepDev sd, const double* __restrict__ dt_src, int flags) {
+    grid_release();
+    grid_wait();
+    const int n = *sd.n_fallback;
+    bool last = blockIdx.x == 0;
+    if (n > 0) {
+        __shared__ int arrived;
+        finalize_deferred<M, N>(m, x_src, x, aux, params, sd, dt_src, flags, n);
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) arrived = atomicAdd(sd.tail_done, 1);
+        __syncthreads();
+        last = arrived == (int)gridDim.x - 1;
+        __threadfence();
+    }
+    if (!last) return;
+    for (int i = threadIdx.x; i < sd.n_inst; i += blockDim.x) {
+        end_instance(sd, i, 1, 0.0, nullptr);
+        begin_instance(sd, i);
+    }
+    if (threadIdx.x == 0 && n > 0) {
+        *sd.n_fallback = 0;
+        *sd.tail_done = 0;
     }
 }
 

@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(THREADS, MINB) stage_kernel(MeshDev m, Opts o,
     double* const rows = sv + 4 * cst;                 // [3 NQ][fst]
     double* const swl = rows + (size_t)2 * NQ * fst;   // [NQ][cst] clamped stage state
     const int tid = threadIdx.x, nt = blockDim.x;
+    grid_release();
     const StageTile tile = tl.tile[blockIdx.x];
     const int n = tile.n, nloc = tile.nloc, nent = tile.nent;
     const bool second = o.order >= 2, lsq = o.gradient == 1;
@@ -161,6 +162,7 @@ __global__ void __launch_bounds__(THREADS, MINB) stage_kernel(MeshDev m, Opts o,
     // ---- the state of the tile and its rings, raw and clamped
     for (int l = tid; l < n; l += nt)
         for (int j = 0; j < K; ++j) srow[j * cst + l] = tl.ord_lf[(size_t)j * C + tile.c0 + l];
+    grid_wait();   // what follows reads the state
     bool changed = false;
     for (int l = tid; l < nloc; l += nt) {
         const int c = l < n ? tile.c0 + l : tl.ext_cell[tile.e0 + l - n];

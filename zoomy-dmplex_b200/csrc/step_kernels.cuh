@@ -68,7 +68,18 @@ struct StepDev {
                                // [6] cells deferred to the generic Newton path (summed over steps)
     int* fallback;             // [C] cells finalize_kernel deferred to finalize_fallback_kernel
     int* n_fallback;           // their count
+    double* dt_last;           // dt of the step taken last
+    int* tail_done;            // blocks of step_tail_kernel that are done (0 between launches)
 };
+
+// Programmatic dependent launch.  A kernel launched with the attribute may
+// start while its predecessor in the stream still runs; grid_wait() returns
+// once the predecessor is complete and its writes are visible (at once in a
+// plain launch), so everything before it may only touch what no kernel of the
+// stream writes (the mesh and its tiles).  grid_release() lets the successor
+// start as soon as every block of this grid has started.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // bits of DBL_MAX: "no cell constrains dt"
 #define ZSME_RATIO_NONE 0x7FEFFFFFFFFFFFFFULL
@@ -1206,9 +1217,7 @@ __global__ void __launch_bounds__(64) mood_kernel(MeshDev m, double* __restrict_
 // --------------------------------------------------------------- step ends
 // begin: each instance's dt for this step from its CFL dt (or the imposed
 // one), clamped to land on t_end; inactive once t >= t_end.
-static __global__ void begin_step_kernel(StepDev sd, int i0, int ni) {
-    const int i = i0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= i0 + ni) return;
+__device__ __forceinline__ void begin_instance(const StepDev& sd, int i) {
     const double t0 = sd.t[i];
     double d0 = sd.dts ? sd.dts[*sd.step_idx] : sd.dt_cfl[i];
     const int act = t0 < sd.t_end;
@@ -1216,18 +1225,33 @@ static __global__ void begin_step_kernel(StepDev sd, int i0, int ni) {
     sd.active[i] = act;
     sd.dt_step[i] = act ? d0 : 0.0;
 }
+static __global__ void begin_step_kernel(StepDev sd, int i0, int ni) {
+    const int i = i0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= i0 + ni) return;
+    begin_instance(sd, i);
+}
+// Before a run of captured steps: the counters of the call at zero, the first
+// step's dt (each step's tail forms the next one's).
+static __global__ void begin_steps_kernel(StepDev sd) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < sd.n_inst) begin_instance(sd, i);
+    if (i == 0) {
+        for (int k = 0; k < 4; ++k) sd.diag[k] = 0;
+        sd.diag[6] = 0;
+        *sd.n_fallback = 0;
+    }
+}
 
 // end: the instance's minimum ratio -> CFL dt (or dt_max when no cell
 // constrains it, VirtualSolver.hpp:354-356); time advance.  mode 1: step end,
 // mode 0: initial dt = max(dt, min_dt) (MUSCLSolver.hpp:103), mode 2: dt
 // into dt_out only (ComputeTimeStep without side effects).
-static __global__ void end_step_kernel(StepDev sd, int i0, int ni, int mode, double min_dt, double* dt_out) {
-    const int i = i0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= i0 + ni) return;
-    const double r = __longlong_as_double((long long)sd.ratio[i]);
+__device__ __forceinline__ void end_instance(const StepDev& sd, int i, int mode, double min_dt, double* dt_out) {
+    const double r = __longlong_as_double((long long)*(volatile unsigned long long*)&sd.ratio[i]);
     sd.ratio[i] = ZSME_RATIO_NONE;
     const double dt = (!isfinite(r) || r >= 0.5 * DBL_MAX) ? sd.dt_max : sd.cfl * r;
     if (mode == 1) {
+        sd.dt_last[i] = sd.dt_step[i];
         if (sd.active[i]) {
             sd.t[i] = sd.t[i] + sd.dt_step[i];
             if (i == 0) *sd.step_idx += 1;
@@ -1238,6 +1262,11 @@ static __global__ void end_step_kernel(StepDev sd, int i0, int ni, int mode, dou
     } else {
         dt_out[i] = dt;
     }
+}
+static __global__ void end_step_kernel(StepDev sd, int i0, int ni, int mode, double min_dt, double* dt_out) {
+    const int i = i0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= i0 + ni) return;
+    end_instance(sd, i, mode, min_dt, dt_out);
 }
 
 // ------------------------------------------------------- layout transforms
