@@ -309,7 +309,7 @@ class Solver final : public SolverBase {
     // A launch that may start while its predecessor drains (grid_wait in the
     // kernel); per-kernel timing keeps the kernels apart.
     template <class... KA, class... A>
-    void launch_chained(void (*k)(KA...), int grid, int block, size_t smem, A... args) {
+    void launch_chained(bool chain, void (*k)(KA...), int grid, int block, size_t smem, A... args) {
         cudaLaunchAttribute attr{};
         attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr.val.programmaticStreamSerializationAllowed = 1;
@@ -319,7 +319,7 @@ class Solver final : public SolverBase {
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream_;
         cfg.attrs = &attr;
-        cfg.numAttrs = profiling_ ? 0 : 1;
+        cfg.numAttrs = chain && !profiling_ ? 1 : 0;
         cudaLaunchKernelEx(&cfg, k, KA(args)...);
     }
 
@@ -401,7 +401,7 @@ class Solver final : public SolverBase {
         const StageWeights sc{(s - 1.) / s, 1. / s, mode == MODE_EULER ? 1.0 : (mode == MODE_FINAL ? s : s - 1.)};
         const int threads = std::min(kStageThreads, P > 1 ? kStageThreads : (st_fst_ + 31) / 32 * 32);
 #define ZSME_STAGE(PP, KK)                                                                                        \
-    launch_chained(stage_kernel<M, N, PP, KK, kStageThreads, kStageBlocks>, tile_n_, threads, stage_smem(P), md_,  \
+    launch_chained(true, stage_kernel<M, N, PP, KK, kStageThreads, kStageBlocks>, tile_n_, threads, stage_smem(P), md_,  \
                    opts_, tl, sc, x_in, aux_.p, params_.p, t_host, t_dev, frac, dt, active, mode, x_out, base)
         if (pm_.K == 3) {
             if (P == 4) ZSME_STAGE(4, 3);
@@ -441,6 +441,11 @@ class Solver final : public SolverBase {
         ZSME_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
         ZSME_CUDA(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device_));
         LaunchConfig lc{128, 128, 128, 128};
+        // finalize's register cap: us per launch on a B200 uncapped and capped, level 4
+        // at 2.0 M cells 459 and 424 (3 blocks of 128; 4: 438), level 2 at 977 k cells
+        // 157 and 119 (4: 124), level 1 at 498 k cells 45.2 and 39.7 (4; 3: 45.2);
+        // level 0 needs no more registers than any cap leaves
+        lc.finalize_occ = NQ >= 8 ? 3 : (NQ >= 6 ? 4 : 1);
         default_tiles(lc);
         if (st_.block_size > 0) lc.prep = lc.face = lc.gather = st_.block_size;
         int rc = set_launch(lc);
@@ -726,7 +731,7 @@ class Solver final : public SolverBase {
         const int C = pm_.C;
         // staging buffer j is free once its copy of two calls ago has left the device
         ZSME_CUDA(cudaStreamWaitEvent(stream_, ev_d2h_[j], 0));
-        soa_to_aos_kernel<<<blocks_for(C, 128), 128, 0, stream_>>>(x_.p, out_stage_[j].p, old_of_new_.p, 0, C, C, NQ);
+        launch_to_aos(x_.p, out_stage_[j].p, 0, C, NQ);
         ZSME_CUDA(cudaGetLastError());
         ZSME_CUDA(cudaEventRecord(ev_out_[j], stream_));
         ZSME_CUDA(cudaStreamWaitEvent(d2h_, ev_out_[j], 0));
@@ -742,10 +747,15 @@ class Solver final : public SolverBase {
         return ZSME_OK;
     }
 
+    // cells [c0, c0 + cn) of nv component rows into caller order
+    void launch_to_aos(const double* soa, double* aos, int c0, int cn, int nv) {
+        soa_to_aos_kernel<<<blocks_for(cn, 128), 128, (size_t)129 * nv * sizeof(double), stream_>>>(
+            soa, aos, old_of_new_.p, c0, cn, pm_.C, nv);
+    }
     int get_soa(int inst, const double* soa, int nv, double* out, bool device) {
         const int c0 = pm_.inst_cell_off[inst], cn = pm_.inst_cell_off[inst + 1] - c0;
         double* dst = device ? out : tmp_b_.p;
-        soa_to_aos_kernel<<<blocks_for(cn, 128), 128, 0, stream_>>>(soa, dst, old_of_new_.p, c0, cn, pm_.C, nv);
+        launch_to_aos(soa, dst, c0, cn, nv);
         ZSME_CUDA(cudaGetLastError());
         if (!device)
             ZSME_CUDA(cudaMemcpyAsync(out, tmp_b_.p, (size_t)nv * cn * sizeof(double), cudaMemcpyDeviceToHost, stream_));
@@ -911,9 +921,17 @@ class Solver final : public SolverBase {
                         const FinalGather* fg = nullptr, const double* x_src = nullptr, bool chained = false) {
         if (!x_src) x_src = x_.p;
         const int gb = blocks_for(cn, lc_.finalize);
+        // Blocks of finalize that start beside the last stage blocks of an SM run under
+        // their shared-memory carve-out, with little L1 for the spilled Newton state:
+        // worth it only where a launch is a large part of the step (us per step early
+        // and not: level 2, 114 k cells 105 and 108; level 4, 2.0 M cells 2608 and 2540)
+        const bool early = tile_n_ <= 4 * kStageBlocks * sm_count_;
         if ((flags & FIN_SOURCE) && !chained) cudaMemsetAsync(sd.n_fallback, 0, sizeof(int), stream_);
         mark(ZSME_KERNEL_FINALIZE, true);
-        if (fg) {
+        if (!(flags & FIN_SOURCE)) {
+            launch_chained(early, finalize_kernel<M, N, 4, false, false>, gb, lc_.finalize, 0, md_, c0, cn, x_src, x_.p,
+                           aux_.p, params_.p, sd, dt_src, flags, FinalGather{});
+        } else if (fg) {
             switch (lc_.finalize_occ) {
 #define ZSME_FING(OCC)                                                                                           \
     case OCC:                                                                                                    \
@@ -928,7 +946,7 @@ class Solver final : public SolverBase {
             switch (lc_.finalize_occ) {
 #define ZSME_FIN(OCC)                                                                                            \
     case OCC:                                                                                                    \
-        launch_chained(finalize_kernel<M, N, OCC>, gb, lc_.finalize, 0, md_, c0, cn, x_src, x_.p, aux_.p,         \
+        launch_chained(early, finalize_kernel<M, N, OCC>, gb, lc_.finalize, 0, md_, c0, cn, x_src, x_.p, aux_.p,         \
                        params_.p, sd, dt_src, flags, FinalGather{});                                             \
         break;
                 ZSME_FIN(2) ZSME_FIN(3) ZSME_FIN(4)
@@ -938,7 +956,7 @@ class Solver final : public SolverBase {
         }
         mark(ZSME_KERNEL_FINALIZE, false);
         if (chained) {
-            launch_chained(step_tail_kernel<M, N>, std::min(blocks_for(cn, 64), 4 * sm_count_), 64, 0, md_, x_src, x_.p,
+            launch_chained(true, step_tail_kernel<M, N>, std::min(blocks_for(cn, 64), 4 * sm_count_), 64, 0, md_, x_src, x_.p,
                            aux_.p, params_.p, sd, dt_src, flags);
             return;
         }

@@ -206,7 +206,7 @@ enum FinalizeFlags {
 // GATHER: the cell's state is the last SSP stage's result, formed here from
 // the face contributions (gather_final_state) instead of read from x_src (x
 // itself, or the last stage's output buffer).
-template <class M, class N, bool GENERIC, bool GATHER = false>
+template <class M, class N, bool GENERIC, bool GATHER = false, bool SOURCE = true>
 __device__ __forceinline__ int finalize_cell(const MeshDev& m, int c, int I, const double* x_src, double* x,
                                              double* __restrict__ aux, const double* p, const StepDev& sd,
                                              const double* __restrict__ dt_src, int flags, double& ratio,
@@ -219,13 +219,15 @@ __device__ __forceinline__ int finalize_cell(const MeshDev& m, int c, int I, con
 #pragma unroll
     for (int i = 0; i < NA; ++i) a[i] = aux[(size_t)i * C + c];
     if (flags & FIN_PRE) constrain<M>(q, a, p);
-    if (flags & FIN_SOURCE) {
-        const int rc = newton_cell<M, GENERIC>(dt_src[I], q, a, p);
-        if constexpr (!GENERIC) {
-            if (rc < 0) return -1;
+    if constexpr (SOURCE) {
+        if (flags & FIN_SOURCE) {
+            const int rc = newton_cell<M, GENERIC>(dt_src[I], q, a, p);
+            if constexpr (!GENERIC) {
+                if (rc < 0) return -1;
+            }
+            if (rc > 0) atomicAdd(&sd.diag[2], 1);
+            if (flags & FIN_PRE) constrain<M>(q, a, p);
         }
-        if (rc > 0) atomicAdd(&sd.diag[2], 1);
-        if (flags & FIN_PRE) constrain<M>(q, a, p);
     }
     if (flags & FIN_POST) constrain<M>(q, a, p);
     if (flags & FIN_WRITE) {
@@ -324,7 +326,7 @@ __device__ __forceinline__ void block_ratio_min(const StepDev& sd, int I, double
 // GATHER: the kernel also performs the last SSP stage's gather (fg), so the
 // stage result never round-trips through x; a deferred cell gets that result
 // written to x for finalize_fallback_kernel.
-template <class M, class N, int MINB, bool GATHER = false>
+template <class M, class N, int MINB, bool GATHER = false, bool SOURCE = true>
 __global__ void __launch_bounds__(128, MINB) finalize_kernel(MeshDev m, int c0, int cn, const double* x_src,
                                                        double* x, double* __restrict__ aux,
                                                        const double* __restrict__ params, StepDev sd, const double* __restrict__ dt_src, int flags,
@@ -338,7 +340,7 @@ __global__ void __launch_bounds__(128, MINB) finalize_kernel(MeshDev m, int c0, 
     double ratio = DBL_MAX;
     const bool act = I >= 0 && (sd.active ? (sd.active[I] != 0) : true);
     bool defer = false;
-    if (act) defer = finalize_cell<M, N, false, GATHER>(m, c, I, x_src, x, aux, params + (size_t)I * m.np, sd, dt_src,
+    if (act) defer = finalize_cell<M, N, false, GATHER, SOURCE>(m, c, I, x_src, x, aux, params + (size_t)I * m.np, sd, dt_src,
                                                          flags, ratio, &fg) < 0;
     if constexpr (GATHER) {
         if (defer) {   // the generic path restarts from the stage result
@@ -348,7 +350,7 @@ __global__ void __launch_bounds__(128, MINB) finalize_kernel(MeshDev m, int c0, 
             for (int i = 0; i < NQ; ++i) x[(size_t)i * m.C + c] = q[i];
         }
     }
-    if (flags & FIN_SOURCE) defer_append(sd, defer, c);
+    if (SOURCE && (flags & FIN_SOURCE)) defer_append(sd, defer, c);
     if (flags & FIN_DT) block_ratio_min(sd, I, ratio);
 }
 

@@ -1317,13 +1317,26 @@ static __global__ void aos_to_soa_kernel(const double* __restrict__ aos, double*
     const int o = old_of_new[c];
     for (int i = 0; i < nq; ++i) soa[(size_t)i * C + c] = aos[(size_t)o * nq + i];
 }
-static __global__ void soa_to_aos_kernel(const double* __restrict__ soa, double* __restrict__ aos,
-                                         const int* __restrict__ old_of_new, int c0, int cn, int C, int nq) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= cn) return;
-    const int c = c0 + r;
-    const int o = old_of_new[c];
-    for (int i = 0; i < nq; ++i) aos[(size_t)o * nq + i] = soa[(size_t)i * C + c];
+// Blocks of 128 cells through shared memory ([nq][129] doubles): the component
+// rows are read coalesced and a cell's components written next to one another,
+// whole sectors of the caller's buffer (one thread per cell wrote one double
+// of a sector at a time: 221 us for 2.0 M cells of 12 components).
+static __global__ void __launch_bounds__(128) soa_to_aos_kernel(const double* __restrict__ soa,
+                                                                double* __restrict__ aos,
+                                                                const int* __restrict__ old_of_new, int c0, int cn,
+                                                                int C, int nq) {
+    extern __shared__ double tile[];
+    __shared__ int old[128];
+    const int r0 = blockIdx.x * 128, n = min(128, cn - r0), t = threadIdx.x;
+    if (t < n) {
+        old[t] = old_of_new[c0 + r0 + t];
+        for (int i = 0; i < nq; ++i) tile[i * 129 + t] = soa[(size_t)i * C + c0 + r0 + t];
+    }
+    __syncthreads();
+    for (int e = t; e < n * nq; e += 128) {
+        const int l = e / nq, i = e - l * nq;
+        aos[(size_t)old[l] * nq + i] = tile[i * 129 + l];
+    }
 }
 
 }  // namespace zsme
