@@ -1159,20 +1159,19 @@ class Solver final : public SolverBase {
         };
         rhs(x_.p, wl0, 0.0, imex_g_[0].p);
         imex_source_kernel<M><<<nb, 128, 0, stream_>>>(md_, x_.p, aux_.p, params_.p, imex_s_[0].p, act);
-        const ImexTerms t1{{imex_g_[0].p}, {imex_s_[0].p}, {K::a10}, {K::t10}, 1};
-        imex_stage_kernel<M><<<blocks_for(C, 64), 64, 0, stream_>>>(md_, t1, x_.p, aux_.p, params_.p, dt, act,
+        const ImexTerms<1> t1{{imex_g_[0].p}, {imex_s_[0].p}, {K::a10}, {K::t10}};
+        imex_stage_kernel<M, 1><<<nb, 128, 0, stream_>>>(md_, t1, x_.p, aux_.p, params_.p, dt, act,
                                                                     imex_y_[0].p, imex_s_[1].p, iscal_.p + 1);
         rhs(imex_y_[0].p, nullptr, K::c1, imex_g_[1].p);
-        const ImexTerms t2{{imex_g_[0].p, imex_g_[1].p}, {imex_s_[0].p, imex_s_[1].p}, {K::a20, K::a21},
-                           {K::t20, K::t21}, 2};
-        imex_stage_kernel<M><<<blocks_for(C, 64), 64, 0, stream_>>>(md_, t2, x_.p, aux_.p, params_.p, dt, act,
+        const ImexTerms<2> t2{{imex_g_[0].p, imex_g_[1].p}, {imex_s_[0].p, imex_s_[1].p}, {K::a20, K::a21},
+                              {K::t20, K::t21}};
+        imex_stage_kernel<M, 2><<<nb, 128, 0, stream_>>>(md_, t2, x_.p, aux_.p, params_.p, dt, act,
                                                                     imex_y_[1].p, imex_s_[2].p, iscal_.p + 1);
         rhs(imex_y_[1].p, nullptr, K::c2, imex_g_[2].p);
-        const ImexTerms tb{{imex_g_[0].p, imex_g_[1].p, imex_g_[2].p},
+        const ImexTerms<3> tb{{imex_g_[0].p, imex_g_[1].p, imex_g_[2].p},
                            {imex_s_[0].p, imex_s_[1].p, imex_s_[2].p},
                            {K::b0, K::b1, K::b2},
-                           {K::b0, K::b1, K::b2},
-                           3};
+                           {K::b0, K::b1, K::b2}};
         imex_final_kernel<M><<<nb, 128, 0, stream_>>>(md_, tb, x_.p, dt, act);
     }
     // ------------------------------------------------ fully implicit strategy
