@@ -85,6 +85,34 @@ def test_rhs_equals_the_separate_kernels(name, gradient, order, limiter):
             g.close()
 
 
+@pytest.mark.parametrize("name", sorted(CASES))
+@pytest.mark.parametrize("gradient", ["green_gauss", "least_squares"])
+@pytest.mark.parametrize("positivity", ["zhang_shu", "mood"])
+def test_positivity_rhs_equals_the_separate_kernels(name, gradient, positivity):
+    c = CASES[name]()
+    kw = dict(gradient=gradient, positivity=positivity)
+    ref = _solver(c, {"tile_faces": 0}, **kw)
+    states = dict(_states(c))
+    want = {k: ref.rhs(q) for k, q in states.items()}
+    for tile in (64, 160, 256):
+        g = _solver(c, {"tile_faces": tile, "fuse_final": 1}, **kw)
+        for k, q in states.items():
+            assert np.array_equal(g.rhs(q), want[k], equal_nan=True), (k, tile)
+        g.close()
+
+
+@pytest.mark.parametrize("order,positivity", [(2, "zhang_shu"), (2, "mood"), (1, "zhang_shu"), (1, "mood")])
+def test_positivity_steps_equal_the_separate_kernels(order, positivity):
+    c = cases.wet_dry_patchwork(24)
+    kw = dict(reconstruction_order=order, positivity=positivity)
+    ref = _solver(c, {"tile_faces": 0}, **kw)
+    g = _solver(c, {"tile_faces": 96, "fuse_final": 1}, **kw)
+    for s in (ref, g):
+        s.step(12)
+    assert np.array_equal(g.get_state(), ref.get_state()) and g.time() == ref.time()
+    assert g.sync().n_mood_cells == ref.sync().n_mood_cells
+
+
 @pytest.mark.parametrize("name", ["l0", "l4", "mixed", "1d"])
 @pytest.mark.parametrize("order,stages", [(1, 2), (2, 2), (2, 3), (2, 5)])
 def test_steps_equal_the_separate_kernels(name, order, stages):

@@ -386,7 +386,8 @@ int build_stage_tiles(const PreparedMesh& p, const FaceTiles& t, int order, bool
                     s.gho_face.push_back(f);
                 }
                 const uint32_t row = fstamp[f] == b ? (uint32_t)frow[f] : kRowNone;
-                s.loc[j * NE + ent] = across | (row << 12) | ((uint32_t)((meta >> 2) & 1) << 23) | ((uint32_t)k << 24);
+                s.loc[j * NE + ent] = across | (row << 12) | ((uint32_t)((meta >> 2) & 1) << 23) | ((uint32_t)k << 24) |
+                                    (1u << 26);
             }
         }
         s.gho_off[b + 1] = (int)s.gho_cell.size();

@@ -81,7 +81,7 @@ struct StageTiles {
 };
 // loc: bits 0-11 local index across the face (kLocNone: none), bits 12-22 the
 // face's row in the tile (kRowNone: not one of the tile's faces), bit 23 the
-// entry is support[0], bits 24-25 the cell's slot of the face
+// entry is support[0], bits 24-25 the cell's slot of the face, bit 26 set
 constexpr uint32_t kLocNone = 0xfff, kRowNone = 0x7ff;
 int build_stage_tiles(const PreparedMesh& p, const FaceTiles& t, int order, bool green_gauss, StageTiles& out);
 

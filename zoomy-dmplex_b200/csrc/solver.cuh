@@ -284,16 +284,9 @@ class Solver final : public SolverBase {
     // shared memory.  us per step on a B200, level 4 at 15.8 k cells: 96 faces
     // and 2 threads per cell 45.1, 256 and 1 56.5; level 2 at 51.2 k cells: 320
     // faces 61.6, 256 71.5, 128 66.1; level 4 at 231 k cells: 256 342, 128 354,
-    // 64 408.  Without it (positivity variants): face + gather tiles of
-    // up to 256 faces, smaller while the mesh would give fewer than three tiles
-    // per SM.
+    // 64 408.
     void default_tiles(LaunchConfig& lc) const {
-        int tf = std::min(256, (int)(kMaxTileSmem / (3 * NQ * sizeof(double))));
-        if (st_.positivity != ZSME_POSITIVITY_NONE) {
-            while (tf > 64 && pm_.F / tf < 3 * sm_count_) tf /= 2;
-            lc.tile_faces = tf;
-            return;
-        }
+        const int tf = std::min(256, (int)(kMaxTileSmem / (3 * NQ * sizeof(double))));
         lc.fuse_final = 1;
         // a tile evaluates about 1 / 0.87 of the faces it owns; its rows take
         // about 1.06 cells and 3 NQ doubles per face
@@ -331,11 +324,20 @@ class Solver final : public SolverBase {
     // with 80: 468 against 414 at 498 k cells, spilling)
     static constexpr int kStageBlocks = NQ >= 6 ? 2 : 3;
     bool wants_stage() const {
-        return lc_.tile_faces > 0 && lc_.fuse_final && st_.positivity == ZSME_POSITIVITY_NONE;
+        // MOOD at order 1 works on x_ between the stage and finalize
+        return lc_.tile_faces > 0 && lc_.fuse_final &&
+               !(st_.positivity == ZSME_POSITIVITY_MOOD && st_.reconstruction_order < 2);
     }
+    // the positivity variants' reconstruction
+    bool well_balanced() const { return st_.positivity != ZSME_POSITIVITY_NONE && st_.reconstruction_order >= 2; }
     // the stage kernel serves the step's stages and right-hand sides
     bool use_stage() const { return wants_stage() && st_built_ == lc_.tile_faces && st_fits_; }
-    int stage_parts() const { return lc_.prep_lean >= 3 ? 4 : (lc_.prep_lean == 2 ? 2 : 1); }
+    int stage_parts() const { return well_balanced() ? 1 : lc_.prep_lean >= 3 ? 4 : (lc_.prep_lean == 2 ? 2 : 1); }
+    template <int KM, int P, bool WB = false>
+    static cudaError_t stage_smem_limit(int bytes) {
+        return cudaFuncSetAttribute(stage_kernel<M, N, P, KM, kStageThreads, kStageBlocks, WB>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    }
     int upload_stage_tiles(const FaceTiles& t) {
         StageTiles s;
         int rc = build_stage_tiles(pm_, t, st_.reconstruction_order, st_.gradient != ZSME_GRADIENT_LSQ, s);
@@ -379,8 +381,10 @@ class Solver final : public SolverBase {
         ZSME_CUDA(cudaGetLastError());
         ZSME_CUDA(cudaStreamSynchronize(stream_));   // a chained launch reads it without waiting for the stream
         const int bytes = (int)kMaxStageSmem;   // a limit of the kernel, shared by every handle
-#define ZSME_STAGE_ATTR(P)                                                                                            ZSME_CUDA(cudaFuncSetAttribute(stage_kernel<M, N, P, 3, kStageThreads, kStageBlocks>,                                                            cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));                              ZSME_CUDA(cudaFuncSetAttribute(stage_kernel<M, N, P, 4, kStageThreads, kStageBlocks>,                                                            cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        ZSME_STAGE_ATTR(1) ZSME_STAGE_ATTR(2) ZSME_STAGE_ATTR(4)
+#define ZSME_STAGE_ATTR(...)                                                                                       \
+    ZSME_CUDA((stage_smem_limit<3, __VA_ARGS__>(bytes)));                                                           \
+    ZSME_CUDA((stage_smem_limit<4, __VA_ARGS__>(bytes)));
+        ZSME_STAGE_ATTR(1) ZSME_STAGE_ATTR(2) ZSME_STAGE_ATTR(4) ZSME_STAGE_ATTR(1, true)
 #undef ZSME_STAGE_ATTR
         return ZSME_OK;
     }
@@ -398,20 +402,22 @@ class Solver final : public SolverBase {
         const StageTilesDev tl{st_tile_.p, tile_in_faces_.p, tile_ord_lf_.p, st_ext_cell_.p, st_gho_cell_.p,
                                st_gho_face_.p, st_loc_.p, st_geo_.p, st_entries_, fst, cst};
         const int s = opts_.stages;
+        const StagePositivity pos{st_.positivity, st_.wet_dry_eps};
         const StageWeights sc{(s - 1.) / s, 1. / s, mode == MODE_EULER ? 1.0 : (mode == MODE_FINAL ? s : s - 1.)};
         const int threads = std::min(kStageThreads, P > 1 ? kStageThreads : (st_fst_ + 31) / 32 * 32);
-#define ZSME_STAGE(PP, KK)                                                                                        \
-    launch_chained(true, stage_kernel<M, N, PP, KK, kStageThreads, kStageBlocks>, tile_n_, threads, stage_smem(P), md_,  \
-                   opts_, tl, sc, x_in, aux_.p, params_.p, t_host, t_dev, frac, dt, active, mode, x_out, base)
-        if (pm_.K == 3) {
-            if (P == 4) ZSME_STAGE(4, 3);
-            else if (P == 2) ZSME_STAGE(2, 3);
-            else ZSME_STAGE(1, 3);
-        } else {
-            if (P == 4) ZSME_STAGE(4, 4);
-            else if (P == 2) ZSME_STAGE(2, 4);
-            else ZSME_STAGE(1, 4);
-        }
+#define ZSME_STAGE(...)                                                                                       \
+    launch_chained(true, stage_kernel<M, N, __VA_ARGS__>, tile_n_, threads, stage_smem(P), md_, opts_, tl, sc, pos, \
+                   x_in, aux_.p, params_.p, t_host, t_dev, frac, dt, active, mode, x_out, base)
+#define ZSME_STAGE_P(KK)                                                                                          \
+    do {                                                                                                          \
+        if (well_balanced()) ZSME_STAGE(1, KK, kStageThreads, kStageBlocks, true);                            \
+        else if (P == 4) ZSME_STAGE(4, KK, kStageThreads, kStageBlocks);                                      \
+        else if (P == 2) ZSME_STAGE(2, KK, kStageThreads, kStageBlocks);                                      \
+        else ZSME_STAGE(1, KK, kStageThreads, kStageBlocks);                                                  \
+    } while (0)
+        if (pm_.K == 3) ZSME_STAGE_P(3);
+        else ZSME_STAGE_P(4);
+#undef ZSME_STAGE_P
 #undef ZSME_STAGE
         mark(ZSME_KERNEL_FLUX, false);
     }

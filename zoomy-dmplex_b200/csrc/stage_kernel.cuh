@@ -34,8 +34,8 @@ struct StageTilesDev {
     const int* gho_face;
     const unsigned* loc;    // [K][entries]
     const double* geo;      // [2 K DIM + 2][entries]: per face the outward normal (Green-Gauss) or the
-                            // weights (least squares), then face centroid - cell centroid (zero off
-                            // the tile), then the volume and its reciprocal
+                            // weights (least squares), then face centroid - cell centroid (zero where
+                            // there is no face), then the volume and its reciprocal
     int entries;
     int fst;                // row length of the face rows (> the most faces of a tile)
     int cst;                // row length of the cell rows (>= the most cells and ghosts of a tile)
@@ -71,6 +71,11 @@ inline size_t stage_smem_doubles(int fst, int cst) {
 struct StageWeights {
     double state, start, dt_div;
 };
+// The positivity variants' reconstruction (prep_wb_kernel): variant and dry threshold.
+struct StagePositivity {
+    int variant;
+    double eps;
+};
 
 // The entries' geometry, gathered once when the tiles are built, so that the
 // stage kernel reads it coalesced and without waiting for indices.
@@ -85,7 +90,7 @@ static __global__ void __launch_bounds__(128) stage_entries_kernel(MeshDev m, co
         const size_t ent = (size_t)t.eo + l;
         for (int k = 0; k < K; ++k) {
             const unsigned e = loc[(size_t)k * NE + ent];
-            const bool across = (e & 0xfffu) != kLocNone, row = ((e >> 12) & 0x7ffu) != kRowNone, isL = (e >> 23) & 1u;
+            const bool across = (e & 0xfffu) != kLocNone, isL = (e >> 23) & 1u, face = (e >> 26) & 1u;
             const int slot = (int)((e >> 24) & 3u), f = m.slot_face[(size_t)slot * C + c];
             for (int d = 0; d < DIM; ++d) {
                 double w = 0.0;
@@ -93,7 +98,7 @@ static __global__ void __launch_bounds__(128) stage_entries_kernel(MeshDev m, co
                 if (across && !least_squares) w = isL ? m.fnr[(size_t)d * m.F + f] : -m.fnr[(size_t)d * m.F + f];
                 geo[((size_t)k * DIM + d) * NE + ent] = w;
                 geo[((size_t)(K + k) * DIM + d) * NE + ent] =
-                    row ? m.slot_dx[((size_t)slot * 2 + d) * C + c] : 0.0;
+                    face ? m.slot_dx[((size_t)slot * 2 + d) * C + c] : 0.0;
             }
         }
         geo[(size_t)2 * K * DIM * NE + ent] = m.vol[c];
@@ -101,11 +106,12 @@ static __global__ void __launch_bounds__(128) stage_entries_kernel(MeshDev m, co
     }
 }
 
+// WB: the face states of the positivity variants (prep_wb_kernel; order 2, P = 1).
 // mode / x_in / x_out / base as gather_kernel, except that x_out never is
 // x_in (another tile reads its rim there): MODE_MID and MODE_EULER write x_out.
-template <class M, class N, int P, int KM, int THREADS, int MINB>
+template <class M, class N, int P, int KM, int THREADS, int MINB, bool WB = false>
 __global__ void __launch_bounds__(THREADS, MINB) stage_kernel(MeshDev m, Opts o, StageTilesDev tl,
-                                                              StageWeights sc,
+                                                              StageWeights sc, StagePositivity pos,
                                                               const double* __restrict__ x_in,
                                                               const double* __restrict__ aux,
                                                               const double* __restrict__ params, double t_host,
@@ -273,6 +279,169 @@ __global__ void __launch_bounds__(THREADS, MINB) stage_kernel(MeshDev m, Opts o,
                 for (int d = 0; d < DIM; ++d) g[d] += geo[k][d] * fv;
             }
         };
+        // the plain gradient, as prep_kernel writes it
+        auto plain_gradient = [&](int i, double (&g)[DIM]) {
+            double q, v[KM];
+            load(sw, i, q, v);
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) g[d] = 0.0;
+#pragma unroll
+            for (int k = 0; k < KM; ++k) {
+                if ((le[k] & 0xfffu) == kLocNone) continue;
+                const double fv = lsq ? v[k] - q : (inner[k] ? 0.5 * (q + v[k]) : v[k]);
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) g[d] += geo[k][d] * fv;
+            }
+#pragma unroll
+            for (int d = 0; d < DIM; ++d)
+                if (divide) g[d] = g[d] / vol;
+        };
+        if constexpr (WB) {
+            static_assert(P == 1, "one thread per cell");
+            constexpr int B = 0, H = 1;
+            const double eps2 = venkat_eps2<DIM>(vol);
+            const double b_bar = sq[B * cst + ent], h_bar = sq[H * cst + ent];
+            // the cell's face states (see prep_wb_kernel for the scheme); plain: with
+            // the divisions prep_wb_kernel makes, for the cells whose branch-free
+            // quotients the other form reports odd
+            auto reconstruct = [&](auto plain) {
+                bool odd = !lsq && !divide;
+                auto gradient_of = [&](int i, double (&g)[DIM]) {
+                    if (plain) {
+                        plain_gradient(i, g);
+                        return;
+                    }
+                    double q, v[KM];
+                    load(sw, i, q, v);
+                    gradient(lsq, whole, q, v, g);
+                    odd |= !whole && exponent_word(q) >= 0x7ff00000u;
+                    if (!lsq) {
+#pragma unroll
+                        for (int e = 0; e < DIM; ++e) g[e] = by_vol.quotient_or(g[e], odd);
+                    }
+                };
+                // Venkatakrishnan factor: the smallest over the cell's faces
+                auto factor = [&](double wc, double wmn, double wmx, const double (&g)[DIM]) {
+                    double ph = 1.0;
+#pragma unroll
+                    for (int k = 0; k < KM; ++k) {
+                        double delta = 0.0;
+#pragma unroll
+                        for (int e = 0; e < DIM; ++e) delta += g[e] * geo[k][DIM + e];
+                        const bool skip = fabs(delta) < 1e-14 || !(le[k] >> 26 & 1u);
+                        const double dm = (delta > 0) ? (wmx - wc) : (wmn - wc);
+                        const double nu = dm * dm + eps2 + 2 * delta * dm;
+                        const double de = dm * dm + 2 * delta * delta + delta * dm + eps2;
+                        double pf;
+                        if (plain) {
+                            pf = (de > 1e-30) ? nu / de : 1.0;
+                        } else {
+                            bool far = !(de > 1e-30);
+                            const RnDivisor by_de(de, rn_reciprocal(de, far));
+                            pf = by_de.quotient_or(nu, far);
+                            odd |= far & !skip;
+                        }
+                        pf = (pf < 1.0) ? pf : 1.0;   // std::min(1, pf)
+                        pf = (0.0 < pf) ? pf : 0.0;   // std::max(0, pf)
+                        ph = !skip && pf < ph ? pf : ph;
+                    }
+                    return ph;
+                };
+                double gb[DIM], ge[DIM], phb, phe;
+                gradient_of(B, gb);
+                gradient_of(H, ge);
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) ge[d] = ge[d] + gb[d];
+                {
+                    double q, vb[KM], vh[KM], mn, mx;
+                    load(sq, B, q, vb);
+                    bounds(whole, q, vb, mn, mx);
+                    phb = factor(q, mn, mx, gb);
+                    load(sq, H, q, vh);
+#pragma unroll
+                    for (int k = 0; k < KM; ++k) vh[k] = vb[k] + vh[k];
+                    bounds(whole, b_bar + h_bar, vh, mn, mx);
+                    phe = factor(b_bar + h_bar, mn, mx, ge);
+                }
+                if (h_bar < pos.eps) phb = phe = 0.0;
+                phb = (phe < phb) ? phe : phb;
+                double sh[DIM];
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) sh[d] = phe * ge[d] - phb * gb[d];
+                double hmin = h_bar;
+#pragma unroll
+                for (int k = 0; k < KM; ++k) {
+                    double hf = h_bar;
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d) hf += sh[d] * geo[k][DIM + d];
+                    if (hf < hmin && (le[k] >> 26 & 1u)) hmin = hf;
+                }
+                double theta = 1.0;
+                if (pos.variant != ZSME_POSITIVITY_MOOD && hmin < 0.0) {
+                    const double gap = h_bar - hmin;
+                    double th = h_bar / ((gap < 1e-14) ? 1e-14 : gap);
+                    th = (th < 1.0) ? th : 1.0;
+                    theta = (0.0 < th) ? th : 0.0;
+                }
+                // effective gradients: b, then eta
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) {
+                    const double gbd = gb[d];
+                    gb[d] = phb * gbd;
+                    ge[d] = phb * gbd + theta * sh[d];
+                }
+                bool dry[KM];
+#pragma unroll
+                for (int k = 0; k < KM; ++k) {
+                    double db = 0.0, de = 0.0;
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d) db += gb[d] * geo[k][DIM + d];
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d) de += ge[d] * geo[k][DIM + d];
+                    const double b_f = b_bar + db;
+                    const double hd = (b_bar + h_bar) + de - b_f;
+                    const double h_f = (hd < 0.0) ? 0.0 : hd;
+                    dry[k] = h_f < pos.eps;
+                    rows[B * fst + fso[k]] = b_f;
+                    rows[H * fst + fso[k]] = h_f;
+                }
+                constexpr int CW = (NQ - 2) % 2 == 0 ? 2 : 1;
+#pragma unroll 1
+                for (int i = 2; i < NQ; i += CW) {
+                    double out[CW][KM];
+#pragma unroll
+                    for (int ii = 0; ii < CW; ++ii) {
+                        double g[DIM], q, v[KM], mn, mx;
+                        gradient_of(i + ii, g);
+                        load(sq, i + ii, q, v);
+                        bounds(whole, q, v, mn, mx);
+                        double ph = factor(q, mn, mx, g);
+                        if (h_bar < pos.eps) ph = 0.0;
+                        ph = (phe < ph) ? phe : ph;
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d) g[d] = theta * ph * g[d];
+#pragma unroll
+                        for (int k = 0; k < KM; ++k) {
+                            double di = 0.0;
+#pragma unroll
+                            for (int d = 0; d < DIM; ++d) di += g[d] * geo[k][DIM + d];
+                            out[ii][k] = dry[k] ? 0.0 : (q + di);
+                        }
+                    }
+#pragma unroll
+                    for (int ii = 0; ii < CW; ++ii)
+#pragma unroll
+                        for (int k = 0; k < KM; ++k) rows[(i + ii) * fst + fso[k]] = out[ii][k];
+                }
+                return odd;
+            };
+            if (reconstruct(std::false_type())) reconstruct(std::true_type());
+            if (live && ent < n) {
+                sv[ent] = vol;
+                sv[cst + ent] = rvol;
+            }
+            continue;
+        }
         bool vac = false;
         if constexpr (NQ > 1) {   // VacuumLimiter: minimum depth over the cell and its neighbours
             double q, v[KM], mn, mx;
@@ -366,32 +535,16 @@ __global__ void __launch_bounds__(THREADS, MINB) stage_kernel(MeshDev m, Opts o,
             odd |= num[k] > 0.0 && !(num[k] >= 0x1p-800);
             al[k] = by_den.quotient_or(num[k], odd);
         }
-        // the plain gradient and limiter, as prep_kernel writes them
-        auto plain_component = [&](int i, double& q, double (&g)[DIM], double& mn, double& mx) {
-            double v[KM];
-            load(sw, i, q, v);
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) g[d] = 0.0;
-#pragma unroll
-            for (int k = 0; k < KM; ++k) {
-                if ((le[k] & 0xfffu) == kLocNone) continue;
-                const double fv = lsq ? v[k] - q : (inner[k] ? 0.5 * (q + v[k]) : v[k]);
-#pragma unroll
-                for (int d = 0; d < DIM; ++d) g[d] += geo[k][d] * fv;
-            }
-#pragma unroll
-            for (int d = 0; d < DIM; ++d)
-                if (divide) g[d] = g[d] / vol;
-            if (clamped) load(swl, i, q, v);
-            bounds(false, q, v, mn, mx);
-        };
+        // an odd cell: the gradient and limiter as prep_kernel writes them
         if (odd && !vac) {
 #pragma unroll
             for (int k = 0; k < KM; ++k) al[k] = 1.0;
 #pragma unroll 1
             for (int ii = 0; ii < NC; ++ii) {
-                double q, g[DIM], mn, mx;
-                plain_component(component(ii), q, g, mn, mx);
+                double q, v[KM], g[DIM], mn, mx;
+                plain_gradient(component(ii), g);
+                load(sq, component(ii), q, v);
+                bounds(false, q, v, mn, mx);
 #pragma unroll 1
                 for (int k = 0; k < KM; ++k) {
                     double d = 0.0;
@@ -458,8 +611,9 @@ __global__ void __launch_bounds__(THREADS, MINB) stage_kernel(MeshDev m, Opts o,
 #pragma unroll 1
             for (int ii = 0; ii < NC; ++ii) {
                 const int i = component(ii);
-                double q, g[DIM], mn, mx;
-                plain_component(i, q, g, mn, mx);
+                double g[DIM];
+                plain_gradient(i, g);
+                const double q = sq[i * cst + ent];
 #pragma unroll
                 for (int k = 0; k < KM; ++k) {
                     double d = 0.0;
