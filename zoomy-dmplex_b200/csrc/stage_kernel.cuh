@@ -164,7 +164,6 @@ __global__ void __launch_bounds__(THREADS, MINB) stage_kernel(MeshDev m, Opts o,
         rvol = g[(2 * K * DIM + 1) * NE];
     };
     geometry();
-
     // ---- the state of the tile and its rings, raw and clamped
     for (int l = tid; l < n; l += nt)
         for (int j = 0; j < K; ++j) srow[j * cst + l] = tl.ord_lf[(size_t)j * C + tile.c0 + l];
@@ -639,7 +638,7 @@ __global__ void __launch_bounds__(THREADS, MINB) stage_kernel(MeshDev m, Opts o,
 
     // ---- sums, / volume and the stage combination (gather_kernel, stage_update),
     // NCG components per thread; consecutive threads, consecutive cells
-    constexpr int NCG = NQ % 3 == 0 ? 3 : (NQ % 4 == 0 ? 4 : 2), G = (NQ + NCG - 1) / NCG;
+    constexpr int NCG = NQ % 4 == 0 ? 4 : (NQ % 3 == 0 ? 3 : 2), G = (NQ + NCG - 1) / NCG;
     static_assert(G * NCG == NQ, "the parts cover the components");
     for (int task = tid; task < n * G; task += nt) {
         const int part = task / n, l = task - part * n;
