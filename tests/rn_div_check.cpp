@@ -38,11 +38,16 @@ int main() {
         if (i % 1004 == 0) b = make(mb, (int)(g() % 2000) - 1000, 0);
         const RnDivisor d(b);
         const double t = a / b;
-        if (!same(d.quotient(a), t) || !same(d.quotient(-a), -t)) return printf("quotient %a / %a\n", a, b), 1;
+        const RnDivisor neg(-b);
+        if (!same(d.quotient(a), t) || !same(d.quotient(-a), -t) || !same(neg.quotient(a), -t))
+            return printf("quotient %a / %a\n", a, b), 1;
         bool odd = false;
         const double q = d.quotient_or(a, odd);
         if (!odd && !same(q, t)) return printf("quotient_or %a / %a\n", a, b), 1;
         odd_n += odd;
+        odd = false;
+        const double qs = neg.signed_quotient_or(a, odd);
+        if (!odd && !same(qs, -t)) return printf("signed_quotient_or %a / %a\n", a, -b), 1;
         odd = false;
         const double y = rn_reciprocal(b, odd);
         if (!odd && !same(y, 1.0 / b)) return printf("rn_reciprocal %a\n", b), 1;

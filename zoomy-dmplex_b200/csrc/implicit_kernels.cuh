@@ -13,6 +13,7 @@
 // (solver.cuh); the vector kernels here serve its GMRES.
 #pragma once
 #include "imex_kernels.cuh"
+#include "rn_div.h"
 
 namespace zsme {
 
@@ -33,15 +34,12 @@ struct BdfTerms {
 };
 
 template <class M>
-__global__ void __launch_bounds__(128) imp_residual_kernel(MeshDev m, const double* __restrict__ y,
-                                                           const double* __restrict__ aux,
-                                                           const double* __restrict__ params,
-                                                           const double* __restrict__ R, BdfTerms b,
-                                                           double* __restrict__ f) {
+__device__ __forceinline__ void imp_residual_cell(const MeshDev& m, int c, const double* __restrict__ y,
+                                                  const double* __restrict__ aux, const double* __restrict__ params,
+                                                  const double* __restrict__ R, const BdfTerms& b,
+                                                  double (&f)[M::n_dof_q]) {
     constexpr int NQ = M::n_dof_q, NA = M::n_dof_qaux;
     const int C = m.C;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
     const double* p = params + (size_t)cell_instance(m, c) * m.np;
     double q[NQ], a[NA], S[NQ];
 #pragma unroll
@@ -50,35 +48,60 @@ __global__ void __launch_bounds__(128) imp_residual_kernel(MeshDev m, const doub
     for (int i = 0; i < NA; ++i) a[i] = aux[(size_t)i * C + c];
     imex_source_cell<M>(q, a, p, S);
     const double c0 = b.coef ? b.coef[0] : b.c0, c1 = b.coef ? b.coef[1] : b.c1;
-    const double c2 = b.coef ? b.coef[2] : b.c2, h = b.coef ? b.coef[3] : b.h;
+    const double c2 = b.coef ? b.coef[2] : b.c2;
+    const RnDivisor by_h(b.coef ? b.coef[3] : b.h);
 #pragma unroll
     for (int i = 0; i < NQ; ++i) {
         const size_t id = (size_t)i * C + c;
-        const double xd = b.xdot ? b.xdot[id] : (c0 * q[i] + c1 * b.xn[id] + c2 * b.xnm1[id]) / h;
-        f[id] = (xd - S[i]) - R[id];
+        const double xd = b.xdot ? b.xdot[id] : by_h.quotient(c0 * q[i] + c1 * b.xn[id] + c2 * b.xnm1[id]);
+        f[i] = (xd - S[i]) - R[id];
     }
 }
+template <class M>
+__global__ void __launch_bounds__(128) imp_residual_kernel(MeshDev m, const double* __restrict__ y,
+                                                           const double* __restrict__ aux,
+                                                           const double* __restrict__ params,
+                                                           const double* __restrict__ R, BdfTerms b,
+                                                           double* __restrict__ f) {
+    constexpr int NQ = M::n_dof_q;
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= m.C) return;
+    double fc[NQ];
+    imp_residual_cell<M>(m, c, y, aux, params, R, b, fc);
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) f[(size_t)i * m.C + c] = fc[i];
+}
 
-// The four forward-difference blocks of one interior face (ComputeFaceJacobian_FD,
-// ModularSolver.hpp:130-185) or the one block of a boundary face with a
-// condition (ComputeBoundaryJacobian_FD, :187-236), each scaled by area /
-// volume of its row's cell.  fj [F][4][NQ][NQ]: LL, LR, RL, RR.  Column j of
-// every block comes from one perturbed evaluation, so no block is held whole.
+// The forward-difference blocks of a face: of an interior one
+// (ComputeFaceJacobian_FD, ModularSolver.hpp:130-185) or the one block of a
+// boundary face with a condition (ComputeBoundaryJacobian_FD, :187-236), each
+// scaled by area / volume of its row's cell.  fj [4][NQ*NQ][F]: LL, LR, RL, RR,
+// faces fastest.  Thread (f, y) perturbs columns of one state, y / kSplit = 0
+// the left one (LL and RL), 1 the right one (LR and RR), y % kSplit its share of
+// the columns.  A face's columns in one thread, its blocks written NQ*NQ doubles
+// apart, took 215 us for 43 k level-2 faces: 24 unpipelined divisions by the step
+// per column and a sector per store.
+constexpr int kJacSplit = 2;
 template <class M, class N>
-__global__ void __launch_bounds__(128) imp_face_jac_kernel(MeshDev m, const double* __restrict__ xl,
+__global__ void __launch_bounds__(128, 3) imp_face_jac_kernel(MeshDev m, const double* __restrict__ xl,
                                                            const double* __restrict__ al,
                                                            const double* __restrict__ params, double t,
                                                            double* __restrict__ fj) {
     constexpr int NQ = M::n_dof_q, NA = M::n_dof_qaux, Q2 = NQ * NQ;
+    constexpr int NJ = (NQ + kJacSplit - 1) / kJacSplit;
     const int F = m.F, C = m.C;
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= F) return;
-    double* out = fj + (size_t)f * 4 * Q2;
+    const int side = blockIdx.y / kJacSplit, j0 = (blockIdx.y % kJacSplit) * NJ, j1 = min(NQ, j0 + NJ);
+    // entry (i, j) of the rows of L and of R
+    double* const rowL = fj + (size_t)(side == 0 ? 0 : 1) * Q2 * F + f;
+    double* const rowR = fj + (size_t)(side == 0 ? 2 : 3) * Q2 * F + f;
     const int L = m.face_L[f], R = m.face_R[f], bc = m.face_bc[f];
     const double area = m.farea[f];
     const bool used = area > 1e-15 && (R >= 0 || bc >= 0);
-    if (!used) {
-        for (int e = 0; e < 4 * Q2; ++e) out[e] = 0.0;
+    if (!used || (R < 0 && side == 1)) {
+        for (int j = j0; j < j1; ++j)
+            for (int i = 0; i < NQ; ++i) rowL[(size_t)(i * NQ + j) * F] = rowR[(size_t)(i * NQ + j) * F] = 0.0;
         return;
     }
     const double* p = params + (size_t)face_instance(m, f) * m.np;
@@ -86,101 +109,76 @@ __global__ void __launch_bounds__(128) imp_face_jac_kernel(MeshDev m, const doub
     const double nh[3] = {m.fn[f], m.fn[F + f], 0.0};
     const double xf[3] = {m.fc[f], m.fc[F + f], 0.0};
     const double eps = implicit_fd::eps;
-    double qL[NQ], aL[NA];
+    const RnDivisor by_eps(eps);
+    double qL[NQ], aL[NA], qR[NQ], aR[NA];
 #pragma unroll
     for (int i = 0; i < NQ; ++i) qL[i] = xl[(size_t)i * C + L];
 #pragma unroll
     for (int i = 0; i < NA; ++i) aL[i] = al[(size_t)i * C + L];
     const double fL = area / m.vol[L];
+    double fR = 0.0;
     if (R >= 0) {
-        double qR[NQ], aR[NA];
 #pragma unroll
         for (int i = 0; i < NQ; ++i) qR[i] = xl[(size_t)i * C + R];
 #pragma unroll
         for (int i = 0; i < NA; ++i) aR[i] = al[(size_t)i * C + R];
-        const double fR = area / m.vol[R];
-        const auto Fb = N::numerical_flux(qL, qR, aL, aR, p, nh);
-        const auto NCb = N::numerical_fluctuations(qL, qR, aL, aR, p, nh);
-        for (int side = 0; side < 2; ++side) {
-            // side 0 perturbs the left state (columns of LL and RL), side 1 the right (LR and RR)
-            double* Jrow0 = out + (side == 0 ? 0 : 1) * Q2;   // LL or LR, rows of L
-            double* Jrow1 = out + (side == 0 ? 2 : 3) * Q2;   // RL or RR, rows of R
-            for (int j = 0; j < NQ; ++j) {
-                double qp[NQ], ap[NA];
-#pragma unroll
-                for (int k = 0; k < NQ; ++k) qp[k] = side == 0 ? qL[k] : qR[k];
-#pragma unroll
-                for (int k = 0; k < NA; ++k) ap[k] = side == 0 ? aL[k] : aR[k];
-                qp[j] += eps;
-                if (NA > 0) {
-                    const auto ra = M::update_aux_variables(qp, ap, p, 0.0, X0);
-#pragma unroll
-                    for (int k = 0; k < NA; ++k) ap[k] = ra[k];
-                }
-                const auto Fp = side == 0 ? N::numerical_flux(qp, qR, ap, aR, p, nh)
-                                          : N::numerical_flux(qL, qp, aL, ap, p, nh);
-                const auto NCp = side == 0 ? N::numerical_fluctuations(qp, qR, ap, aR, p, nh)
-                                           : N::numerical_fluctuations(qL, qp, aL, ap, p, nh);
-#pragma unroll
-                for (int i = 0; i < NQ; ++i) {
-                    const double dFlux = (Fp[i] - Fb[i]) / eps;
-                    double j0 = 0.0, j1 = 0.0;
-                    j0 += dFlux;
-                    j1 -= dFlux;
-                    j0 += (NCp[NQ + i] - NCb[NQ + i]) / eps;
-                    j1 += (NCp[i] - NCb[i]) / eps;
-                    Jrow0[i * NQ + j] = j0 * fL;
-                    Jrow1[i * NQ + j] = j1 * fR;
-                }
-            }
-        }
+        fR = area / m.vol[R];
     } else {
-        double qRb[NQ], aRb[NA];
-        {
-            const auto r = M::boundary_conditions(bc, qL, aL, p, nh, xf, t, 0.0);
+        const auto r = M::boundary_conditions(bc, qL, aL, p, nh, xf, t, 0.0);
 #pragma unroll
-            for (int i = 0; i < NQ; ++i) qRb[i] = r[i];
-            if (NA > 0) {
-                const auto ra = M::update_aux_variables(qRb, aL, p, t, xf);
+        for (int i = 0; i < NQ; ++i) qR[i] = r[i];
+        if (NA > 0) {
+            const auto ra = M::update_aux_variables(qR, aL, p, t, xf);
 #pragma unroll
-                for (int k = 0; k < NA; ++k) aRb[k] = ra[k];
+            for (int k = 0; k < NA; ++k) aR[k] = ra[k];
+        }
+    }
+    const auto Fb = N::numerical_flux(qL, qR, aL, aR, p, nh);
+    const auto NCb = N::numerical_fluctuations(qL, qR, aL, aR, p, nh);
+#pragma unroll 1
+    for (int j = j0; j < j1; ++j) {
+        double pL[NQ], pR[NQ], bL[NA], bR[NA];
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) {
+            pL[k] = side == 0 && k == j ? qL[k] + eps : qL[k];
+            pR[k] = side == 1 && k == j ? qR[k] + eps : qR[k];
+        }
+#pragma unroll
+        for (int k = 0; k < NA; ++k) { bL[k] = aL[k]; bR[k] = aR[k]; }
+        if (NA > 0) {   // the perturbed state's aux
+            if (side == 0) {
+                const auto ra = M::update_aux_variables(pL, bL, p, R >= 0 ? 0.0 : t, R >= 0 ? X0 : xf);
+#pragma unroll
+                for (int k = 0; k < NA; ++k) bL[k] = ra[k];
+            } else {
+                const auto ra = M::update_aux_variables(pR, bR, p, 0.0, X0);
+#pragma unroll
+                for (int k = 0; k < NA; ++k) bR[k] = ra[k];
             }
         }
-        const auto Fb = N::numerical_flux(qL, qRb, aL, aRb, p, nh);
-        const auto NCb = N::numerical_fluctuations(qL, qRb, aL, aRb, p, nh);
-        for (int j = 0; j < NQ; ++j) {
-            double qp[NQ], ap[NA], qr[NQ], ar[NA];
+        if (R < 0) {
+            const auto r = M::boundary_conditions(bc, pL, bL, p, nh, xf, t, 0.0);
 #pragma unroll
-            for (int k = 0; k < NQ; ++k) qp[k] = qL[k];
-#pragma unroll
-            for (int k = 0; k < NA; ++k) ap[k] = aL[k];
-            qp[j] += eps;
+            for (int k = 0; k < NQ; ++k) pR[k] = r[k];
             if (NA > 0) {
-                const auto ra = M::update_aux_variables(qp, ap, p, t, xf);
+                const auto ra = M::update_aux_variables(pR, bL, p, t, xf);
 #pragma unroll
-                for (int k = 0; k < NA; ++k) ap[k] = ra[k];
-            }
-            {
-                const auto r = M::boundary_conditions(bc, qp, ap, p, nh, xf, t, 0.0);
-#pragma unroll
-                for (int k = 0; k < NQ; ++k) qr[k] = r[k];
-            }
-            if (NA > 0) {
-                const auto ra = M::update_aux_variables(qr, ap, p, t, xf);
-#pragma unroll
-                for (int k = 0; k < NA; ++k) ar[k] = ra[k];
-            }
-            const auto Fp = N::numerical_flux(qp, qr, ap, ar, p, nh);
-            const auto NCp = N::numerical_fluctuations(qp, qr, ap, ar, p, nh);
-#pragma unroll
-            for (int i = 0; i < NQ; ++i) {
-                double j0 = 0.0;
-                j0 += (Fp[i] - Fb[i]) / eps;
-                j0 += (NCp[NQ + i] - NCb[NQ + i]) / eps;
-                out[i * NQ + j] = j0 * fL;
+                for (int k = 0; k < NA; ++k) bR[k] = ra[k];
             }
         }
-        for (int e = Q2; e < 4 * Q2; ++e) out[e] = 0.0;
+        const auto Fp = N::numerical_flux(pL, pR, bL, bR, p, nh);
+        const auto NCp = N::numerical_fluctuations(pL, pR, bL, bR, p, nh);
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+            const double dFlux = by_eps.quotient(Fp[i] - Fb[i]);
+            double eL = 0.0, eR = 0.0;
+            eL += dFlux;
+            eR -= dFlux;
+            eL += by_eps.quotient(NCp[NQ + i] - NCb[NQ + i]);
+            eR += by_eps.quotient(NCp[i] - NCb[i]);
+            rowL[(size_t)(i * NQ + j) * F] = eL * fL;
+            rowR[(size_t)(i * NQ + j) * F] = R >= 0 ? eR * fR : 0.0;
+        }
     }
 }
 
@@ -203,10 +201,14 @@ __global__ void __launch_bounds__(64) imp_cell_jac_kernel(MeshDev m, const doubl
     const double* p = params + (size_t)cell_instance(m, c) * m.np;
     const double X0[3] = {0.0, 0.0, 0.0};
     double q[NQ], aux[NA], J[Q2];
+#pragma unroll
     for (int i = 0; i < NQ; ++i) q[i] = xl[(size_t)i * C + c];
+#pragma unroll
     for (int i = 0; i < NA; ++i) aux[i] = al[(size_t)i * C + c];
     if (NQ > 1 && q[1] < implicit_fd::dry_jacobian) {
+#pragma unroll
         for (int e = 0; e < Q2; ++e) J[e] = 0.0;
+#pragma unroll
         for (int i = 0; i < NQ; ++i) J[i * NQ + i] = a;
     } else {
         const auto dSdQ = M::source_jacobian_wrt_variables(q, aux, p);
@@ -214,22 +216,29 @@ __global__ void __launch_bounds__(64) imp_cell_jac_kernel(MeshDev m, const doubl
         double dAdQ[NA * NQ + 1];
         if constexpr (HasAuxJacobian<M>::value) {
             const auto r = M::update_aux_variables_jacobian_wrt_variables(q, aux, p);
+#pragma unroll
             for (int e = 0; e < NA * NQ; ++e) dAdQ[e] = r[e];
         } else {   // forward differences, SourceStep.hpp:16-53
             const auto a0 = M::update_aux_variables(q, aux, p, 0.0, X0);
+#pragma unroll
             for (int j = 0; j < NQ; ++j) {
                 double qp[NQ];
+#pragma unroll
                 for (int mm = 0; mm < NQ; ++mm) qp[mm] = q[mm];
                 const double hh = 1e-7 * (fabs(q[j]) + 1e-7);
                 qp[j] += hh;
                 const auto a1 = M::update_aux_variables(qp, aux, p, 0.0, X0);
+#pragma unroll
                 for (int k = 0; k < NA; ++k) dAdQ[k * NQ + j] = (a1[k] - a0[k]) / hh;
             }
         }
+#pragma unroll
         for (int i = 0; i < NQ; ++i)
+#pragma unroll
             for (int j = 0; j < NQ; ++j) {
                 const double val = i == j ? a : 0.0;
                 double dSource = dSdQ[i * NQ + j];
+#pragma unroll
                 for (int k = 0; k < NA; ++k) dSource += dSdA[i * NA + k] * dAdQ[k * NQ + j];
                 J[i * NQ + j] = val - dSource;
             }
@@ -244,82 +253,148 @@ __global__ void __launch_bounds__(64) imp_cell_jac_kernel(MeshDev m, const doubl
         if (f < 0) continue;
         if (m.face_R[f] < 0 && m.face_bc[f] < 0) continue;
         if (!(m.farea[f] > 1e-15)) continue;
-        blk[nblk++] = fj + ((size_t)f * 4 + (m.face_L[f] == c ? 0 : 3)) * Q2;
+        const double* const here = fj + (size_t)(m.face_L[f] == c ? 0 : 3) * Q2 * m.F + f;
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            if (b == nblk) blk[b] = here;
+        ++nblk;
     }
+#pragma unroll
     for (int e = 0; e < Q2; ++e) {
         double acc = 0.0;
         acc += J[e];
-        for (int b = 0; b < nblk; ++b) acc += blk[b][e];
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            if (b < nblk) acc += blk[b][(size_t)e * m.F];
         pd[(size_t)e * C + c] = acc;
     }
 }
 
 // LU factors of every diagonal block with partial pivoting (the block-Jacobi
-// preconditioner of the Krylov solve): lu in the layout of pd, piv [NQ][C];
-// bad[c] = 1 where a pivot is zero or not finite (that block is applied as the
-// identity).
+// preconditioner of the Krylov solve): lu [NQ*NQ][C] with the row swaps of piv
+// [NQ][C], and the reciprocals of the diagonal in rdiag [NQ][C]; a block with a
+// zero or non-finite pivot is applied as the identity.  Every index is known at
+// compile time, so an 8 x 8 block stays in registers, and a column divides by
+// its pivot's reciprocal.
 template <int NQ>
 __global__ void __launch_bounds__(64) imp_block_lu_kernel(int C, const double* __restrict__ pd,
-                                                          double* __restrict__ lu, int* __restrict__ piv) {
+                                                          double* __restrict__ lu, int* __restrict__ piv,
+                                                          double* __restrict__ rdiag) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
-    double A[NQ * NQ];
-    for (int e = 0; e < NQ * NQ; ++e) A[e] = pd[(size_t)e * C + c];
+    double A[NQ][NQ];
+#pragma unroll
+    for (int i = 0; i < NQ; ++i)
+#pragma unroll
+        for (int j = 0; j < NQ; ++j) A[i][j] = pd[(size_t)(i * NQ + j) * C + c];
     int pv[NQ];
     bool ok = true;
+#pragma unroll
     for (int k = 0; k < NQ; ++k) {
         int mr = k;
-        double mv = fabs(A[k * NQ + k]);
+        double mv = fabs(A[k][k]);
+#pragma unroll
         for (int i = k + 1; i < NQ; ++i) {
-            const double v = fabs(A[i * NQ + k]);
+            const double v = fabs(A[i][k]);
             if (v > mv) { mv = v; mr = i; }
         }
         pv[k] = mr;
-        if (mr != k)
-            for (int j = 0; j < NQ; ++j) {
-                const double tt = A[k * NQ + j];
-                A[k * NQ + j] = A[mr * NQ + j];
-                A[mr * NQ + j] = tt;
-            }
-        const double pkk = A[k * NQ + k];
-        if (!(mv > 0.0) || !isfinite(pkk)) { ok = false; break; }
+        if (mr != k) {
+#pragma unroll
+            for (int i = k + 1; i < NQ; ++i)
+                if (mr == i) {
+#pragma unroll
+                    for (int j = 0; j < NQ; ++j) {
+                        const double tt = A[k][j];
+                        A[k][j] = A[i][j];
+                        A[i][j] = tt;
+                    }
+                }
+        }
+        const double pkk = A[k][k];
+        if (!(mv > 0.0) || !isfinite(pkk)) ok = false;
+        const RnDivisor by_pivot(pkk);
+#pragma unroll
         for (int i = k + 1; i < NQ; ++i) {
-            const double l = A[i * NQ + k] / pkk;
-            A[i * NQ + k] = l;
-            for (int j = k + 1; j < NQ; ++j) A[i * NQ + j] -= l * A[k * NQ + j];
+            const double l = by_pivot.quotient(A[i][k]);
+            A[i][k] = l;
+#pragma unroll
+            for (int j = k + 1; j < NQ; ++j) A[i][j] -= l * A[k][j];
         }
     }
-    if (!ok) {
-        for (int e = 0; e < NQ * NQ; ++e) A[e] = 0.0;
-        for (int i = 0; i < NQ; ++i) { A[i * NQ + i] = 1.0; pv[i] = i; }
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+#pragma unroll
+        for (int j = 0; j < NQ; ++j) lu[(size_t)(i * NQ + j) * C + c] = ok ? A[i][j] : (i == j ? 1.0 : 0.0);
+        piv[(size_t)i * C + c] = ok ? pv[i] : i;
+        rdiag[(size_t)i * C + c] = ok ? 1.0 / A[i][i] : 1.0;
     }
-    for (int e = 0; e < NQ * NQ; ++e) lu[(size_t)e * C + c] = A[e];
-    for (int i = 0; i < NQ; ++i) piv[(size_t)i * C + c] = pv[i];
 }
 
-// z = D^-1 r per cell from the LU factors (r and z may alias)
+// b <- D^-1 b for cell c from the LU factors: each triangle is loaded before it
+// is used, since the row swaps' branches would keep the loads apart, and the
+// quotients are branch-free with a plain repetition behind them.
+template <int NQ>
+__device__ __forceinline__ void imp_block_solve(int C, int c, const double* __restrict__ lu,
+                                                const int* __restrict__ piv, const double* __restrict__ rdiag,
+                                                double (&b)[NQ]) {
+    double T[NQ][NQ], rd[NQ], f[NQ];
+    int pv[NQ];
+    bool swaps = false;
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) pv[k] = piv[(size_t)k * C + c];
+#pragma unroll
+    for (int i = 1; i < NQ; ++i)
+#pragma unroll
+        for (int j = 0; j < i; ++j) T[i][j] = lu[(size_t)(i * NQ + j) * C + c];
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) swaps |= pv[k] != k;
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+        if (swaps) {
+#pragma unroll
+            for (int i = k + 1; i < NQ; ++i) {
+                const double bk = b[k], bi = b[i];
+                b[k] = pv[k] == i ? bi : bk;
+                b[i] = pv[k] == i ? bk : bi;
+            }
+        }
+#pragma unroll
+        for (int i = k + 1; i < NQ; ++i) b[i] -= T[i][k] * b[k];
+    }
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+#pragma unroll
+        for (int j = i; j < NQ; ++j) T[i][j] = lu[(size_t)(i * NQ + j) * C + c];
+        rd[i] = rdiag[(size_t)i * C + c];
+        f[i] = b[i];
+    }
+    auto back = [&](auto plain) {
+        bool odd = false;
+#pragma unroll
+        for (int i = NQ - 1; i >= 0; --i) {
+            double s = f[i];
+#pragma unroll
+            for (int j = i + 1; j < NQ; ++j) s -= T[i][j] * b[j];
+            b[i] = plain ? s / T[i][i] : RnDivisor(T[i][i], rd[i]).signed_quotient_or(s, odd);
+        }
+        return odd;
+    };
+    if (back(std::false_type())) back(std::true_type());
+}
+// z = D^-1 r (r and z may alias)
 template <int NQ>
 __global__ void __launch_bounds__(128) imp_block_solve_kernel(int C, const double* __restrict__ lu,
-                                                              const int* __restrict__ piv, const double* r,
+                                                              const int* __restrict__ piv,
+                                                              const double* __restrict__ rdiag, const double* r,
                                                               double* z) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     double b[NQ];
+#pragma unroll
     for (int i = 0; i < NQ; ++i) b[i] = r[(size_t)i * C + c];
-    for (int k = 0; k < NQ; ++k) {
-        const int mr = piv[(size_t)k * C + c];
-        if (mr != k) {
-            const double tt = b[k];
-            b[k] = b[mr];
-            b[mr] = tt;
-        }
-        for (int i = k + 1; i < NQ; ++i) b[i] -= lu[(size_t)(i * NQ + k) * C + c] * b[k];
-    }
-    for (int i = NQ - 1; i >= 0; --i) {
-        double s = b[i];
-        for (int j = i + 1; j < NQ; ++j) s -= lu[(size_t)(i * NQ + j) * C + c] * b[j];
-        b[i] = s / lu[(size_t)(i * NQ + i) * C + c];
-    }
+    imp_block_solve<NQ>(C, c, lu, piv, rdiag, b);
+#pragma unroll
     for (int i = 0; i < NQ; ++i) z[(size_t)i * C + c] = b[i];
 }
 
@@ -347,45 +422,44 @@ __global__ void __launch_bounds__(128) imp_update_state_kernel(MeshDev m, const 
     for (int i = 0; i < NA; ++i) al[(size_t)i * C + c] = a[i];
 }
 
-// ------------------------------------------------------------ vector kernels
-// The matrix-free Jacobian's differencing parameter from the device dot v.v:
-// hv = sqrt(eps) sqrt(1 + |X|) / |v| (0 for a zero vector)
-static __global__ void imp_hv_kernel(const double* __restrict__ vv, const double* __restrict__ xnorm,
-                                     double* __restrict__ hv) {
-    const double vn = sqrt(*vv);
-    *hv = vn > 0.0 ? 1.4901161193847656e-08 * sqrt(1.0 + *xnorm) / vn : 0.0;
+// out = D^-1 (F(y) - F0) / hv for the perturbed state y = X + hv v whose transport
+// right-hand side is R: the residual, the matrix-free Jacobian's difference
+// quotient (zero when hv is zero) and the block solve of a cell in one pass
+// (29 us as three kernels for 29 k level-2 cells).
+template <class M>
+__global__ void __launch_bounds__(128) imp_apply_kernel(MeshDev m, const double* __restrict__ y,
+                                                        const double* __restrict__ aux,
+                                                        const double* __restrict__ params,
+                                                        const double* __restrict__ R, BdfTerms b,
+                                                        const double* __restrict__ F0, const double* __restrict__ hv,
+                                                        const double* __restrict__ lu, const int* __restrict__ piv,
+                                                        const double* __restrict__ rdiag, double* __restrict__ out) {
+    constexpr int NQ = M::n_dof_q;
+    grid_release();
+    grid_wait();
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, C = m.C;
+    if (c >= C) return;
+    double f[NQ];
+    imp_residual_cell<M>(m, c, y, aux, params, R, b, f);
+    const double h = *hv;
+    const RnDivisor by_h(h);
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) f[i] = h != 0.0 ? by_h.quotient(f[i] - F0[(size_t)i * C + c]) : 0.0;
+    imp_block_solve<NQ>(C, c, lu, piv, rdiag, f);
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) out[(size_t)i * C + c] = f[i];
 }
+
+// ------------------------------------------------------------ vector kernels
 static __global__ void imp_sqrt_kernel(const double* __restrict__ in, double* __restrict__ out) { *out = sqrt(*in); }
 // out = 1.0 x + hv v, hv a device scalar
 static __global__ void imp_perturb_kernel(long long n, const double* __restrict__ x, const double* __restrict__ v,
                                           const double* __restrict__ hv, double* __restrict__ out) {
+    grid_release();
+    grid_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     out[i] = 1.0 * x[i] + *hv * v[i];
-}
-// out = (ft - f0) / hv, zero when hv is zero
-static __global__ void imp_diffquot_dev_kernel(long long n, const double* __restrict__ ft,
-                                               const double* __restrict__ f0, const double* __restrict__ hv,
-                                               double* __restrict__ out) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double h = *hv;
-    out[i] = h != 0.0 ? (ft[i] - f0[i]) / h : 0.0;
-}
-// out = (1.0 / sqrt(ww)) w where ww = w.w > 0 (the next Arnoldi vector)
-static __global__ void imp_normalize_kernel(long long n, const double* __restrict__ ww, const double* __restrict__ w,
-                                            double* __restrict__ out) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double hn = sqrt(*ww);
-    if (hn > 0.0) out[i] = (1.0 / hn) * w[i];
-}
-// out = (ft - f0) / h (the matrix-free Jacobian's difference quotient)
-static __global__ void imp_diffquot_kernel(long long n, const double* __restrict__ ft, const double* __restrict__ f0,
-                                           double h, double* __restrict__ out) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    out[i] = (ft[i] - f0[i]) / h;
 }
 // out = a x + b y (out may alias x or y; y may be null when b = 0)
 static __global__ void imp_lincomb_kernel(long long n, double a, const double* x, double b, const double* y,
@@ -395,52 +469,143 @@ static __global__ void imp_lincomb_kernel(long long n, double a, const double* x
     out[i] = y ? a * x[i] + b * y[i] : a * x[i];
 }
 
-// partial[k][blk] = sum over the block's entries of V_k . w, k < nk (V_k =
-// V + k ld); a fixed tree per block, so the sums are deterministic
-static __global__ void __launch_bounds__(256) imp_multi_dot_kernel(long long n, int nk, const double* __restrict__ V,
-                                                                   long long ld, const double* __restrict__ w,
-                                                                   double* __restrict__ partial) {
-    // grid (nb, nk): block (b, k) takes vector k's chunk b
-    __shared__ double sh[256];
-    const int nb = gridDim.x, k = blockIdx.y;
-    if (k >= nk) return;
-    const double* v = V + (size_t)k * ld;
-    double s = 0.0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)nb * blockDim.x)
-        s += v[i] * w[i];
-    sh[threadIdx.x] = s;
+// Inner products, deterministic: block b sums its chunk (a fixed stride per
+// thread, a fixed tree per block) into partial[k][b], and the last block to
+// arrive sums the partials the same way into out[k].  count: blocks arrived,
+// zero between launches.  hv, when given: the matrix-free Jacobian's
+// differencing parameter sqrt(eps) sqrt(1 + |X|) / |v| from out[0] = v.v (0 for
+// a zero vector).
+struct DotSink {
+    double* partial;
+    int* count;
+    double* out;
+    double* hv;
+    const double* xnorm;
+};
+// the sum of the block's 256 values of s, in thread 0: pairs 128, 64, ... 1 apart
+__device__ __forceinline__ double imp_block_sum(double s, double* sh) {
+    const int t = threadIdx.x;
+    sh[t] = s;
     __syncthreads();
-    for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-        if (threadIdx.x < off) sh[threadIdx.x] += sh[threadIdx.x + off];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) partial[(size_t)k * nb + blockIdx.x] = sh[0];
-}
-// out[k] = sum of partial[k][0 .. nb): one block of 256 threads per k, each
-// thread a fixed stride of the partials, then a fixed tree (deterministic)
-static __global__ void __launch_bounds__(256) imp_reduce_kernel(int nk, int nb, const double* __restrict__ partial,
-                                                                double* __restrict__ out) {
-    __shared__ double sh[256];
-    const int k = blockIdx.x;
-    if (k >= nk) return;
-    double s = 0.0;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) s += partial[(size_t)k * nb + b];
-    sh[threadIdx.x] = s;
+    if (t < 128) sh[t] = s = s + sh[t + 128];
     __syncthreads();
-    for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-        if (threadIdx.x < off) sh[threadIdx.x] += sh[threadIdx.x + off];
-        __syncthreads();
+    if (t < 64) sh[t] = s = s + sh[t + 64];
+    __syncthreads();
+    if (t < 32) {
+        s = s + sh[t + 32];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) s = s + __shfl_down_sync(0xffffffffu, s, off);
     }
-    if (threadIdx.x == 0) out[k] = sh[0];
+    return s;
 }
-// w -= sum_k h_k V_k (classical Gram-Schmidt projection, h on the device)
-static __global__ void imp_multi_axpy_kernel(long long n, int nk, const double* __restrict__ V, long long ld,
-                                             const double* __restrict__ h, double* __restrict__ w) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double s = w[i];
-    for (int k = 0; k < nk; ++k) s -= h[k] * V[(size_t)k * ld + i];
-    w[i] = s;
+// vectors k0 .. k0 + NK (below nk); group: their counter
+template <int NK>
+__device__ __forceinline__ void imp_finish_dots(const double (&s)[NK], int k0, int nk, int group, const DotSink& d) {
+    __shared__ double sh[NK][256];
+    __shared__ int arrived;
+    const int nb = gridDim.x;
+    double block[NK];
+#pragma unroll
+    for (int q = 0; q < NK; ++q) block[q] = imp_block_sum(s[q], sh[q]);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < NK; ++q)
+            if (k0 + q < nk) d.partial[(size_t)(k0 + q) * nb + blockIdx.x] = block[q];
+        __threadfence();
+        arrived = atomicAdd(d.count + group, 1);
+    }
+    __syncthreads();
+    if (arrived != nb - 1) return;
+    __threadfence();
+    double t[NK];
+#pragma unroll
+    for (int q = 0; q < NK; ++q) {
+        t[q] = 0.0;
+        if (k0 + q < nk)
+            for (int b = threadIdx.x; b < nb; b += blockDim.x) t[q] += __ldcg(d.partial + (size_t)(k0 + q) * nb + b);
+    }
+#pragma unroll
+    for (int q = 0; q < NK; ++q) {
+        const double sum = imp_block_sum(t[q], sh[q]);
+        if (threadIdx.x == 0 && k0 + q < nk) {
+            d.out[k0 + q] = sum;
+            if (d.hv && k0 + q == 0) {
+                const double vn = sqrt(sum);
+                *d.hv = vn > 0.0 ? 1.4901161193847656e-08 * sqrt(1.0 + *d.xnorm) / vn : 0.0;
+            }
+        }
+    }
+    if (threadIdx.x == 0) d.count[group] = 0;
+}
+// out[k] = V_k . w, k < nk (V_k = V + k ld): NK vectors per block row
+template <int NK>
+__global__ void __launch_bounds__(256) imp_multi_dot_kernel(long long n, int nk, const double* __restrict__ V,
+                                                            long long ld, const double* __restrict__ w, DotSink d) {
+    grid_release();
+    grid_wait();
+    const int k0 = blockIdx.y * NK;
+    double s[NK];
+    const double* v[NK];
+#pragma unroll
+    for (int q = 0; q < NK; ++q) {
+        s[q] = 0.0;
+        v[q] = V + (size_t)min(k0 + q, nk - 1) * ld;
+    }
+#pragma unroll 2
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x) {
+        const double wi = w[i];
+#pragma unroll
+        for (int q = 0; q < NK; ++q) s[q] += v[q][i] * wi;
+    }
+    imp_finish_dots<NK>(s, k0, nk, blockIdx.y, d);
+}
+// w -= sum_k h_k V_k (classical Gram-Schmidt projection, h on the device) and
+// out[0] = w.w; four elements' chains run side by side
+static __global__ void __launch_bounds__(256) imp_project_kernel(long long n, int nk, const double* __restrict__ V,
+                                                                 long long ld, const double* __restrict__ h,
+                                                                 double* __restrict__ w, DotSink d) {
+    grid_release();
+    grid_wait();
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    double sum[1] = {0.0};
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * stride) {
+        double s[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[e] = i + e * stride < n ? w[i + e * stride] : 0.0;
+#pragma unroll 4
+        for (int k = 0; k < nk; ++k) {
+            const double hk = h[k];
+            const double* const v = V + (size_t)k * ld + i;
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (i + e * stride < n) s[e] -= hk * v[e * stride];
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (i + e * stride < n) {
+                w[i + e * stride] = s[e];
+                sum[0] += s[e] * s[e];
+            }
+    }
+    imp_finish_dots<1>(sum, 0, 1, 0, d);
+}
+// v = (1.0 / sqrt(ww)) w where ww = w.w > 0 (the next Arnoldi vector) and out[0] = v.v
+static __global__ void __launch_bounds__(256) imp_normalize_kernel(long long n, const double* __restrict__ ww,
+                                                                   const double* __restrict__ w,
+                                                                   double* __restrict__ v, DotSink d) {
+    grid_release();
+    grid_wait();
+    const double hn = sqrt(*ww), r = 1.0 / hn;
+    double sum[1] = {0.0};
+#pragma unroll 4
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x) {
+        const double s = hn > 0.0 ? r * w[i] : v[i];
+        v[i] = s;
+        sum[0] += s * s;
+    }
+    imp_finish_dots<1>(sum, 0, 1, 0, d);
 }
 // x += sum_k y_k V_k (the Krylov update, y on the device)
 static __global__ void imp_multi_add_kernel(long long n, int nk, const double* __restrict__ V, long long ld,

@@ -71,21 +71,21 @@ ZSME_RNDIV_FN double rn_reciprocal(double b, bool& odd) {
 
 struct RnDivisor {
     double b, y;
-    // the plain division serves every quotient where b is not in [2^-100, 2^100)
+    // the plain division serves every quotient where |b| is not in [2^-100, 2^100)
     bool fast;
     ZSME_RNDIV_FN explicit RnDivisor(double div)
-        : b(div), y(1.0 / div), fast(div > 0.0 && exponent_word(div) - (923u << 20) < (200u << 20)) {}
+        : b(div), y(1.0 / div), fast(exponent_word(div) - (923u << 20) < (200u << 20)) {}
     ZSME_RNDIV_FN RnDivisor(double div, double reciprocal)   // reciprocal: 1 / div, formed before
-        : b(div), y(reciprocal), fast(div > 0.0 && exponent_word(div) - (923u << 20) < (200u << 20)) {}
+        : b(div), y(reciprocal), fast(exponent_word(div) - (923u << 20) < (200u << 20)) {}
     ZSME_RNDIV_FN double quotient(double a) const {
         const double q0 = a * y;
         const double q1 = rn_fma(rn_fma(-b, q0, a), y, q0);
         double q = rn_fma(rn_fma(-b, q1, a), y, q1);
-        // |a| outside [2^-900, 2^900): q is not to be trusted; a zero keeps its sign (b > 0)
-        if (!fast || exponent_word(a) - (123u << 20) >= (1800u << 20)) q = (fast && a == 0.0) ? a : a / b;
+        // |a| outside [2^-900, 2^900): q is not to be trusted; of a zero, q0 has the sign
+        if (!fast || exponent_word(a) - (123u << 20) >= (1800u << 20)) q = (fast && a == 0.0) ? q0 : a / b;
         return q;
     }
-    // The same without a branch, for a that is never a negative zero: where the
+    // The same without a branch, for b > 0 and an a that is never a negative zero: where the
     // five operations do not give the quotient, odd is set and the caller
     // divides again.
     ZSME_RNDIV_FN double quotient_or(double a, bool& odd) const {
@@ -94,6 +94,11 @@ struct RnDivisor {
         const uint32_t e = exponent_word(a);
         odd |= !fast | ((e - (123u << 20) >= (1800u << 20)) & ((e | lower_word(a)) != 0u));
         return rn_fma(rn_fma(-b, q1, a), y, q1);
+    }
+    // quotient_or for any b and a
+    ZSME_RNDIV_FN double signed_quotient_or(double a, bool& odd) const {
+        const double q = quotient_or(a, odd);
+        return a == 0.0 ? a * y : q;
     }
 };
 

@@ -91,11 +91,12 @@ class Solver final : public SolverBase {
     // residual at zero, restart residual; clamped state and its aux; the
     // assembled diagonal blocks, their LU factors and pivots; the face blocks
     DevBuf<double> imp_xn_, imp_xnm1_, imp_F_, imp_Ft_, imp_xt_, imp_R_, imp_V_, imp_w_, imp_d_, imp_r0_, imp_r_;
-    DevBuf<double> imp_xl_, imp_al_, imp_pd_, imp_lu_, imp_fj_, imp_part_, imp_red_;
+    DevBuf<double> imp_xl_, imp_al_, imp_pd_, imp_lu_, imp_rdiag_, imp_fj_, imp_part_, imp_red_;
     // device scalars of the step: [0] t_{n+1}, [1] |X|, [2..5] BDF c0, c1, c2, h,
-    // [6] v.v, [7] differencing parameter, [8] w.w, [9] X.X
+    // [6] v.v, [7] differencing parameter, [9] X.X
     DevBuf<double> imp_scal_;
-    DevBuf<int> imp_piv_;
+    DevBuf<int> imp_piv_, imp_count_;
+    double* imp_host_ = nullptr;   // page-locked: the projections and w.w of an Arnoldi step
     cudaGraphExec_t imp_graph_[kImpRestart] = {};   // Arnoldi step j, captured on first use
     bool imp_have_prev_ = false;   // a previous implicit step exists: BDF2
     double imp_h_prev_ = 0.0;
@@ -158,6 +159,7 @@ class Solver final : public SolverBase {
     ~Solver() override {
         if (graph_) cudaGraphExecDestroy(graph_);
         imp_drop_graphs();
+        if (imp_host_) cudaFreeHost(imp_host_);
         for (auto e : ev_pool_) cudaEventDestroy(e);
         if (h2d_) {
             cudaStreamSynchronize(h2d_);
@@ -302,12 +304,12 @@ class Solver final : public SolverBase {
     // A launch that may start while its predecessor drains (grid_wait in the
     // kernel); per-kernel timing keeps the kernels apart.
     template <class... KA, class... A>
-    void launch_chained(bool chain, void (*k)(KA...), int grid, int block, size_t smem, A... args) {
+    void launch_chained(bool chain, void (*k)(KA...), dim3 grid, int block, size_t smem, A... args) {
         cudaLaunchAttribute attr{};
         attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr.val.programmaticStreamSerializationAllowed = 1;
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(grid);
+        cfg.gridDim = grid;
         cfg.blockDim = dim3(block);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream_;
@@ -503,6 +505,10 @@ class Solver final : public SolverBase {
             ZSME_CUDA(imp_pd_.alloc((size_t)NQ * NQ * C));
             ZSME_CUDA(imp_lu_.alloc((size_t)NQ * NQ * C));
             ZSME_CUDA(imp_piv_.alloc((size_t)NQ * C));
+            ZSME_CUDA(imp_rdiag_.alloc((size_t)NQ * C));
+            ZSME_CUDA(imp_count_.alloc((size_t)kImpRestart + 1));
+            ZSME_CUDA(cudaMemsetAsync(imp_count_.p, 0, imp_count_.n * sizeof(int), stream_));
+            if (!imp_host_) ZSME_CUDA(cudaMallocHost((void**)&imp_host_, (kImpRestart + 2) * sizeof(double)));
             ZSME_CUDA(imp_fj_.alloc((size_t)4 * NQ * NQ * F));
             ZSME_CUDA(imp_part_.alloc((size_t)(kImpRestart + 1) * imp_dot_blocks()));
             ZSME_CUDA(imp_red_.alloc((size_t)kImpRestart + 8));
@@ -1187,18 +1193,26 @@ class Solver final : public SolverBase {
     int imp_dot_blocks() const { return std::max(1, std::min(2 * sm_count_, blocks_for((long long)NQ * pm_.C, 256))); }
     long long imp_n() const { return (long long)NQ * pm_.C; }
     // V_k . w for k < nk into dev (device; imp_red_ by default) and out (host,
-    // when given: a synchronisation)
-    int imp_dots(const double* V, long long ld, int nk, const double* w, double* out, double* dev = nullptr) {
-        const int nb = imp_dot_blocks();
+    // when given: a synchronisation); hv: the differencing parameter from the
+    // first product, into imp_scal_[7]
+    int imp_dots(const double* V, long long ld, int nk, const double* w, double* out, double* dev = nullptr,
+                 bool hv = false) {
         if (!dev) dev = imp_red_.p;
-        imp_multi_dot_kernel<<<dim3(nb, nk), 256, 0, stream_>>>(imp_n(), nk, V, ld, w, imp_part_.p);
-        imp_reduce_kernel<<<nk, 256, 0, stream_>>>(nk, nb, imp_part_.p, dev);
+        if (nk == 1)
+            launch_chained(true, imp_multi_dot_kernel<1>, dim3(imp_dot_blocks()), 256, 0, imp_n(), nk, V, ld, w,
+                           imp_sink(dev, hv));
+        else
+            launch_chained(true, imp_multi_dot_kernel<4>, dim3(imp_dot_blocks(), (nk + 3) / 4), 256, 0, imp_n(), nk, V, ld,
+                           w, imp_sink(dev, hv));
         ZSME_CUDA(cudaGetLastError());
         if (out) {
             ZSME_CUDA(cudaMemcpyAsync(out, dev, nk * sizeof(double), cudaMemcpyDeviceToHost, stream_));
             ZSME_CUDA(cudaStreamSynchronize(stream_));
         }
         return ZSME_OK;
+    }
+    DotSink imp_sink(double* out, bool hv = false) {
+        return DotSink{imp_part_.p, imp_count_.p, out, hv ? imp_scal_.p + 7 : nullptr, imp_scal_.p + 1};
     }
     int imp_norm(const double* w, double& out) {
         double d = 0.0;
@@ -1234,36 +1248,37 @@ class Solver final : public SolverBase {
         const int C = pm_.C, F = pm_.F;
         imp_update_state_kernel<M><<<blocks_for(C, 128), 128, 0, stream_>>>(md_, y, aux_.p, params_.p, imp_xl_.p,
                                                                           imp_al_.p);
-        imp_face_jac_kernel<M, N><<<blocks_for(F, 128), 128, 0, stream_>>>(md_, imp_xl_.p, imp_al_.p, params_.p, t,
+        imp_face_jac_kernel<M, N><<<dim3(blocks_for(F, 128), 2 * kJacSplit), 128, 0, stream_>>>(md_, imp_xl_.p, imp_al_.p, params_.p, t,
                                                                           imp_fj_.p);
         imp_cell_jac_kernel<M><<<blocks_for(C, 64), 64, 0, stream_>>>(md_, imp_xl_.p, imp_al_.p, params_.p, a,
                                                                       imp_fj_.p, imp_pd_.p);
     }
     // out = D^-1 (F(X + hv v) - F(X)) / hv, hv = sqrt(eps) sqrt(1 + |X|) / |v| (the
     // Walker-Pernice differencing parameter of PETSc's matrix-free Jacobian);
-    // |X|, |v| and hv stay on the device
+    // |X|, |v| and hv stay on the device, hv already in imp_scal_[7]
     void imp_apply(const double* v, double* out) {
         const long long n = imp_n();
-        double* sc = imp_scal_.p;
-        imp_dots(v, 0, 1, v, nullptr, sc + 6);
-        imp_hv_kernel<<<1, 1, 0, stream_>>>(sc + 6, sc + 1, sc + 7);
-        imp_perturb_kernel<<<blocks_for(n, 256), 256, 0, stream_>>>(n, x_.p, v, sc + 7, imp_xt_.p);
-        imp_residual_step(imp_xt_.p, imp_Ft_.p);
-        imp_diffquot_dev_kernel<<<blocks_for(n, 256), 256, 0, stream_>>>(n, imp_Ft_.p, imp_F_.p, sc + 7, out);
-        imp_block_solve_kernel<NQ><<<blocks_for(pm_.C, 128), 128, 0, stream_>>>(pm_.C, imp_lu_.p, imp_piv_.p, out, out);
+        double* hv = imp_scal_.p + 7;
+        launch_chained(true, imp_perturb_kernel, dim3(blocks_for(n, 256)), 256, 0, n, x_.p, v, hv, imp_xt_.p);
+        launch_rhs(imp_xt_.p, nullptr, 0.0, imp_scal_.p, 0.0, imp_R_.p, nullptr, nullptr);
+        launch_chained(true, imp_apply_kernel<M>, dim3(blocks_for(pm_.C, 128)), 128, 0, md_, imp_xt_.p, aux_.p, params_.p,
+                       imp_R_.p, imp_bdf(), imp_F_.p, hv, imp_lu_.p, imp_piv_.p, imp_rdiag_.p, out);
     }
-    // Arnoldi step j: w = D^-1 J V_j, h = V_0..j . w (into imp_red_), w -= V h,
-    // w.w (imp_scal_[8]), V_{j+1} = w / |w|.  Fixed pointers and device
-    // scalars only, so it is captured once per handle as a CUDA graph.
+    // Arnoldi step j, whose differencing parameter is formed: w = D^-1 J V_j, h =
+    // V_0..j . w (into imp_red_), w -= V h, w.w (into imp_red_[j + 1]), V_{j+1} =
+    // w / |w| with its differencing parameter, h and w.w to the host.  Fixed
+    // pointers and device scalars only, so it is captured once per handle as a
+    // CUDA graph.
     void imp_enqueue_arnoldi(int j) {
         const long long n = imp_n();
-        double* w = imp_w_.p;
+        const int nb = imp_dot_blocks();
+        double *w = imp_w_.p, *ww = imp_red_.p + j + 1;
         imp_apply(imp_V_.p + (size_t)j * n, w);
         imp_dots(imp_V_.p, n, j + 1, w, nullptr);
-        imp_multi_axpy_kernel<<<blocks_for(n, 256), 256, 0, stream_>>>(n, j + 1, imp_V_.p, n, imp_red_.p, w);
-        imp_dots(w, 0, 1, w, nullptr, imp_scal_.p + 8);
-        imp_normalize_kernel<<<blocks_for(n, 256), 256, 0, stream_>>>(n, imp_scal_.p + 8, w,
-                                                                      imp_V_.p + (size_t)(j + 1) * n);
+        launch_chained(true, imp_project_kernel, dim3(nb), 256, 0, n, j + 1, imp_V_.p, n, imp_red_.p, w, imp_sink(ww));
+        launch_chained(true, imp_normalize_kernel, dim3(nb), 256, 0, n, ww, w, imp_V_.p + (size_t)(j + 1) * n,
+                       imp_sink(imp_scal_.p + 6, true));
+        cudaMemcpyAsync(imp_host_, imp_red_.p, (j + 2) * sizeof(double), cudaMemcpyDeviceToHost, stream_);
     }
     int imp_arnoldi(int j) {
         if (profiling_) {   // per-kernel timing records events: plain launches
@@ -1294,17 +1309,19 @@ class Solver final : public SolverBase {
         its = 0;
         ZSME_CUDA(cudaMemsetAsync(imp_d_.p, 0, n * sizeof(double), stream_));
         imp_lincomb(-1.0, imp_F_.p, 0.0, nullptr, imp_r0_.p);
-        imp_block_solve_kernel<NQ><<<blocks_for(C, 128), 128, 0, stream_>>>(C, imp_lu_.p, imp_piv_.p, imp_r0_.p,
-                                                                            imp_r0_.p);
+        imp_block_solve_kernel<NQ><<<blocks_for(C, 128), 128, 0, stream_>>>(C, imp_lu_.p, imp_piv_.p, imp_rdiag_.p,
+                                                                            imp_r0_.p, imp_r0_.p);
         double beta = 0.0;
         int rc = imp_norm(imp_r0_.p, beta);
         if (rc) return rc;
         if (!(beta > 0.0)) return ZSME_OK;
         const double tol = std::max(1e-5 * beta, 1e-50);
         const double* r = imp_r0_.p;
-        std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), y(m), hcol(m + 1);
+        std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), y(m);
+        const double* hcol = imp_host_;
         while (true) {
             imp_lincomb(1.0 / beta, r, 0.0, nullptr, imp_V_.p);
+            if ((rc = imp_dots(imp_V_.p, 0, 1, imp_V_.p, nullptr, imp_scal_.p + 6, true))) return rc;
             std::fill(g.begin(), g.end(), 0.0);
             g[0] = beta;
             int j = 0;
@@ -1312,11 +1329,8 @@ class Solver final : public SolverBase {
             for (; j < m;) {
                 // one synchronisation per Arnoldi step: the projections and |w|^2 come back together
                 if ((rc = imp_arnoldi(j))) return rc;
-                double hn2 = 0.0;
-                ZSME_CUDA(cudaMemcpyAsync(hcol.data(), imp_red_.p, (j + 1) * sizeof(double), cudaMemcpyDeviceToHost,
-                                          stream_));
-                ZSME_CUDA(cudaMemcpyAsync(&hn2, imp_scal_.p + 8, sizeof(double), cudaMemcpyDeviceToHost, stream_));
                 ZSME_CUDA(cudaStreamSynchronize(stream_));
+                const double hn2 = hcol[j + 1];
                 const double hn = std::sqrt(hn2);
                 for (int i = 0; i <= j; ++i) H[(size_t)i * m + j] = hcol[i];
                 H[(size_t)(j + 1) * m + j] = hn;
@@ -1352,6 +1366,7 @@ class Solver final : public SolverBase {
             ZSME_CUDA(cudaGetLastError());
             if (done) break;
             // restart: r = D^-1 (-F) - D^-1 J d
+            if ((rc = imp_dots(imp_d_.p, 0, 1, imp_d_.p, nullptr, imp_scal_.p + 6, true))) return rc;
             imp_apply(imp_d_.p, imp_w_.p);
             imp_lincomb(1.0, imp_r0_.p, -1.0, imp_w_.p, imp_r_.p);
             r = imp_r_.p;
@@ -1403,7 +1418,7 @@ class Solver final : public SolverBase {
             imp_sqrt_kernel<<<1, 1, 0, stream_>>>(imp_scal_.p + 9, imp_scal_.p + 1);   // |X| for the differencing
             imp_assemble(t1, x_.p, shift);
             imp_block_lu_kernel<NQ><<<blocks_for(pm_.C, 64), 64, 0, stream_>>>(pm_.C, imp_pd_.p, imp_lu_.p,
-                                                                              imp_piv_.p);
+                                                                              imp_piv_.p, imp_rdiag_.p);
             int gm = 0;
             if ((rc = imp_gmres(gm))) return rc;
             gm_total += gm;
@@ -1514,8 +1529,8 @@ class Solver final : public SolverBase {
                 const bool interior = pm_.face_R[f] >= 0 && pm_.farea[f] > 1e-15;
                 for (int e = 0; e < Q2; ++e) {
                     // the matrix entry: zero plus the one block added there
-                    offdiag[((size_t)o * 2 + 0) * Q2 + e] = interior ? 0.0 + fj[((size_t)f * 4 + 1) * Q2 + e] : 0.0;
-                    offdiag[((size_t)o * 2 + 1) * Q2 + e] = interior ? 0.0 + fj[((size_t)f * 4 + 2) * Q2 + e] : 0.0;
+                    offdiag[((size_t)o * 2 + 0) * Q2 + e] = interior ? 0.0 + fj[((size_t)Q2 + e) * F + f] : 0.0;
+                    offdiag[((size_t)o * 2 + 1) * Q2 + e] = interior ? 0.0 + fj[((size_t)2 * Q2 + e) * F + f] : 0.0;
                 }
             }
         return ZSME_OK;
