@@ -50,7 +50,10 @@ int main() {
         if (!odd && !same(qs, -t)) return printf("signed_quotient_or %a / %a\n", a, -b), 1;
         odd = false;
         const double y = rn_reciprocal(b, odd);
-        if (!odd && !same(y, 1.0 / b)) return printf("rn_reciprocal %a\n", b), 1;
+        bool odd_neg = false;
+        const double yn = rn_reciprocal(-b, odd_neg);
+        if (odd_neg != odd || (!odd && (!same(y, 1.0 / b) || !same(yn, -1.0 / b))))
+            return printf("rn_reciprocal %a\n", b), 1;
         ++n;
     }
     printf("checked %ld odd %ld\n", n, odd_n);

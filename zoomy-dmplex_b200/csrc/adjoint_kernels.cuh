@@ -42,13 +42,16 @@
 // the segment replays run beside the reverse sweep on a second stream, so
 // resident blocks decide the time).  Replays plus reverse sweep per step:
 // caps 4 / 4 / 2 0.285 ms; 4 / 5 / 2 0.283; 4 / 4 / 3 0.287; 3 / 3 / 2 0.308;
-// 5 / 5 / 2 0.303; 6 / 6 / 2 0.327; 2 / 2 / 2 0.330.  The gradients are the
-// same bit for bit under every cap.
+// 5 / 5 / 2 0.303; 6 / 6 / 2 0.327; 2 / 2 / 2 0.330.  With the volume quotients
+// of rn_div.h and the replays on the separate face kernels: 4 / 4 / 2 0.288,
+// 4 / 5 / 2 0.282 (40 steps, the first replay included); launching the reverse
+// kernels programmatically dependent costs 0.02, since they then hold the SMs
+// the replays run on.  The gradients are the same bit for bit under every cap.
 #ifndef ZSME_ADJ_FACE_MINB
 #define ZSME_ADJ_FACE_MINB 4
 #endif
 #ifndef ZSME_ADJ_CELL_MINB
-#define ZSME_ADJ_CELL_MINB 4
+#define ZSME_ADJ_CELL_MINB 5
 #endif
 #ifndef ZSME_ADJ_FIN_MINB
 #define ZSME_ADJ_FIN_MINB 2
@@ -291,19 +294,19 @@ __global__ void __launch_bounds__(128, ZSME_ADJ_FACE_MINB) adj_face_vjp_kernel(M
     const double dt = *dtp;
     const double scale = factor * dt;
     const double vL = m.vol[L], vR = R >= 0 ? m.vol[R] : 0.0;
-    double w[3 * NQ];
+    double w[3 * NQ], muL[NQ], muR[NQ];
 #pragma unroll
     for (int i = 0; i < NQ; ++i) {
-        double muL = scale * v[(size_t)i * C + L];
-        if (vL > 1e-15) muL /= vL;
-        double muR = 0.0;
-        if (R >= 0) {
-            muR = scale * v[(size_t)i * C + R];
-            if (vR > 1e-15) muR /= vR;
-        }
-        w[i] = (muR - muL) * area;
-        w[NQ + i] = -(area * muR);
-        w[2 * NQ + i] = -(area * muL);
+        muL[i] = scale * v[(size_t)i * C + L];
+        muR[i] = R >= 0 ? scale * v[(size_t)i * C + R] : 0.0;
+    }
+    if (vL > 1e-15) divide_all(muL, vL);
+    if (vR > 1e-15) divide_all(muR, vR);
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+        w[i] = (muR[i] - muL[i]) * area;
+        w[NQ + i] = -(area * muR[i]);
+        w[2 * NQ + i] = -(area * muL[i]);
     }
     const double nh[3] = {m.fn[f], m.fn[F + f], 0.0};
     const double xf[3] = {m.fc[f], m.fc[F + f], 0.0};
@@ -472,10 +475,7 @@ __global__ void __launch_bounds__(128, ZSME_ADJ_CELL_MINB) adj_cell_kernel(MeshD
                 }
             }
             const double vol = m.vol[c];
-            if (vol > 1e-15) {
-#pragma unroll
-                for (int i = 0; i < NQ * DIM; ++i) g[i] /= vol;
-            }
+            if (vol > 1e-15) divide_all(g, vol);
         }
         // the forward limiter, remembering which branch set each face's alpha
 #pragma unroll
@@ -599,10 +599,7 @@ __global__ void __launch_bounds__(128, ZSME_ADJ_CELL_MINB) adj_cell_kernel(MeshD
         }
     } else {
         const double vol = m.vol[c];
-        if (vol > 1e-15) {
-#pragma unroll
-            for (int i = 0; i < NQ * DIM; ++i) gam[i] /= vol;
-        }
+        if (vol > 1e-15) divide_all(gam, vol);
 #pragma unroll
         for (int k = 0; k < KM; ++k) {
             if (ff[k] < 0) continue;

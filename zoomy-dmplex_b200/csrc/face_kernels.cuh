@@ -115,17 +115,14 @@ __global__ void __launch_bounds__(128, MINB) face_kernel(MeshDev m, int f0, int 
 // stage combination of PETSc's TSSSP "rks2" for cell c of instance I, whose
 // summed face contributions are acc.
 template <class M>
-__device__ __forceinline__ void stage_update(const MeshDev& m, const Opts& o, int c, int I, double* acc, int mode,
+__device__ __forceinline__ void stage_update(const MeshDev& m, const Opts& o, int c, int I, double (&acc)[M::n_dof_q], int mode,
                                              const double* x_in, double* x_out, double* base,
                                              const double* __restrict__ dt_step, const double* __restrict__ aux,
                                              const double* __restrict__ params, double* __restrict__ xl_out) {
     constexpr int NQ = M::n_dof_q;
     const int C = m.C;
     const double v = m.vol[c];
-    if (v > 1e-15) {
-#pragma unroll
-        for (int i = 0; i < NQ; ++i) acc[i] /= v;
-    }
+    if (v > 1e-15) divide_all(acc, v);
     const double h = dt_step ? dt_step[I] : 0.0;
     const int s = o.stages;
     switch (mode) {
@@ -213,10 +210,7 @@ __device__ __forceinline__ void gather_final_state(const MeshDev& m, int c, int 
         }
     }
     const double v = m.vol[c];
-    if (v > 1e-15) {
-#pragma unroll
-        for (int i = 0; i < NQ; ++i) acc[i] /= v;
-    }
+    if (v > 1e-15) divide_all(acc, v);
     const int s = fg.stages;
     const double h = fg.dt_step[I];
     const double al = (s - 1.) / s, be = h / s, ga = 1. / s;

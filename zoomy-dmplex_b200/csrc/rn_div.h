@@ -51,7 +51,7 @@ ZSME_RNDIV_FN double rn_fma(double a, double b, double c) {
 #endif
 }
 
-// RN(1 / b) for b in [2^-100, 2^100) without a branch: Newton-Raphson from a
+// RN(1 / b) for |b| in [2^-100, 2^100) without a branch: Newton-Raphson from a
 // seed good to 2^-18 or better (two steps reach half an ulp and a bit, the
 // third rounds correctly by Markstein's theorem on reciprocals, which leaves
 // out the significand of all ones).  odd is set where b is outside that range
@@ -63,7 +63,7 @@ ZSME_RNDIV_FN double rn_reciprocal(double b, bool& odd) {
 #else
     double y = (double)(1.0f / (float)b) * (1.0 + 0x1p-19);
 #endif
-    odd |= (exponent_word(b) - (923u << 20) >= (200u << 20)) | (lower_word(b) == 0xffffffffu) | !(b > 0.0);
+    odd |= (exponent_word(b) - (923u << 20) >= (200u << 20)) | (lower_word(b) == 0xffffffffu);
     y = rn_fma(rn_fma(-b, y, 1.0), y, y);
     y = rn_fma(rn_fma(-b, y, 1.0), y, y);
     return rn_fma(rn_fma(-b, y, 1.0), y, y);
@@ -101,5 +101,27 @@ struct RnDivisor {
         return a == 0.0 ? a * y : q;
     }
 };
+
+// a[i] /= b for every i
+template <int N>
+ZSME_RNDIV_FN void divide_all(double (&a)[N], double b) {
+    const RnDivisor by(b);
+    bool odd = false;
+    double q[N];
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (int i = 0; i < N; ++i) q[i] = by.signed_quotient_or(a[i], odd);
+    if (odd) {
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+        for (int i = 0; i < N; ++i) q[i] = a[i] / b;
+    }
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (int i = 0; i < N; ++i) a[i] = q[i];
+}
 
 }  // namespace zsme

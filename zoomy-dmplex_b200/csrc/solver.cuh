@@ -137,6 +137,10 @@ class Solver final : public SolverBase {
     cudaStream_t adj_side_ = nullptr;
     int adj_par_ = 0, adj_tape_steps_ = 0;
     const double* adj_aux_cur_ = nullptr;
+    // the segments' captured graphs (replay, reverse per tape buffer), kept while
+    // everything they address stays the same (adj_key_)
+    cudaGraphExec_t adj_gx_[4] = {};
+    std::vector<const void*> adj_key_;
     bool adj_overlapped_ = false;  // the last zsme_adjoint overlapped its replays with the reverse sweep
     double adj_phase_ms_[3] = {0, 0, 0};  // last zsme_adjoint: forward pass, replays, reverse sweep
     MeshDev md_{};
@@ -159,6 +163,7 @@ class Solver final : public SolverBase {
     ~Solver() override {
         if (graph_) cudaGraphExecDestroy(graph_);
         imp_drop_graphs();
+        adj_drop_graphs();
         if (imp_host_) cudaFreeHost(imp_host_);
         for (auto e : ev_pool_) cudaEventDestroy(e);
         if (h2d_) {
@@ -243,6 +248,7 @@ class Solver final : public SolverBase {
             graph_ = nullptr;
         }
         imp_drop_graphs();
+        adj_drop_graphs();
         if (ready_) return ensure_tiles();
         return ZSME_OK;
     }
@@ -454,6 +460,9 @@ class Solver final : public SolverBase {
         // 157 and 119 (4: 124), level 1 at 498 k cells 45.2 and 39.7 (4; 3: 45.2);
         // level 0 needs no more registers than any cap leaves
         lc.finalize_occ = NQ >= 8 ? 3 : (NQ >= 6 ? 4 : 1);
+        // the separate face kernel's (adjoint replays): level 4, us per launch at 2.0 M
+        // cells, 3 blocks per SM 350, uncapped 407; level 2 the same within 2 %
+        lc.face_occ = NQ >= 10 ? 3 : 4;
         default_tiles(lc);
         if (st_.block_size > 0) lc.prep = lc.face = lc.gather = st_.block_size;
         int rc = set_launch(lc);
@@ -886,7 +895,10 @@ class Solver final : public SolverBase {
     void launch_flux(int mode, double t_host, const double* t_dev, double frac, const double* x_in, double* x_out,
                      double* base, const double* dt, const int* active, double* xl_out = nullptr,
                      bool face_only = false) {
-        if (lc_.tile_faces > 0) {   // fused face + gather over tiles
+        // fused face + gather over tiles; a handle on the whole-stage kernel comes here
+        // for the adjoint's replays alone, where the separate kernels are as fast at
+        // level 1 (104 and 103 us per step, 79 k cells) and faster above
+        if (lc_.tile_faces > 0 && !use_stage()) {
             mark(ZSME_KERNEL_FLUX, true);
             const TilesDev tl{tile_cell_off_.p, tile_face_off_.p, tile_in_off_.p, tile_in_faces_.p, tile_ord_lf_.p,
                               tile_stride_};
@@ -1728,6 +1740,14 @@ class Solver final : public SolverBase {
             enqueue_step(adj_seg_dt_.p + par, x_.p, tp);
         }
     }
+    void adj_drop_graphs() {
+        for (auto& g : adj_gx_)
+            if (g) {
+                cudaGraphExecDestroy(g);
+                g = nullptr;
+            }
+        adj_key_.clear();
+    }
     void adj_reverse(int cnt) {
         for (int k = cnt - 1; k >= 0; --k) adj_step(k);
     }
@@ -1896,14 +1916,21 @@ class Solver final : public SolverBase {
                                                       adj_oseed_.p + first[NS], C, adj_lam0_.p);
         }
         const bool graphs = !profiling_;
-        cudaGraphExec_t gx[4] = {nullptr, nullptr, nullptr, nullptr};   // replay, reverse per tape buffer
-        struct GraphGuard {
-            cudaGraphExec_t* g;
-            ~GraphGuard() {
-                for (int i = 0; i < 4; ++i)
-                    if (g[i]) cudaGraphExecDestroy(g[i]);
+        // replay and reverse per tape buffer; a handle's next call with the same
+        // intervals and buffers launches the graphs of this one
+        cudaGraphExec_t* const gx = adj_gx_;
+        {
+            std::vector<const void*> key = {(const void*)(size_t)E, (const void*)(size_t)overlap,
+                                            (const void*)(size_t)tape_steps, adj_tape_.p, adj_aux_snap_.p, adj_lam0_.p,
+                                            adj_lam1_.p, adj_lam2_.p, adj_own_w_.p, adj_own_wl_.p, adj_wl_.p,
+                                            adj_out_w_.p, adj_out_wl_.p, adj_gfs_.p, adj_lp_cell_.p, adj_lp_.p,
+                                            adj_seg_dt_.p, adj_seg_t_.p, adj_seg_n0_.p, adj_first_.p, adj_ocell_.p,
+                                            adj_ocomp_.p, adj_oseed_.p, adj_dts_.p, adj_th_.p};
+            if (key != adj_key_) {
+                adj_drop_graphs();
+                adj_key_ = key;
             }
-        } graph_guard{gx};
+        }
         auto capture = [&](cudaGraphExec_t* out, bool replay) -> int {
             cudaGraph_t gr = nullptr;
             ZSME_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
@@ -1974,7 +2001,8 @@ class Solver final : public SolverBase {
             for (int par = 0; par < 2; ++par) {
                 adj_par_ = par;
                 adj_aux_cur_ = adj_aux_snap_.p + (size_t)par * na;
-                if ((rc = capture(&gx[par], true)) || (rc = capture(&gx[2 + par], false))) return rc;
+                if (!gx[par] && (rc = capture(&gx[par], true))) return rc;
+                if (!gx[2 + par] && (rc = capture(&gx[2 + par], false))) return rc;
             }
             cudaEvent_t ov[5];   // replay done (2), reverse done (2), start
             int made = 0;

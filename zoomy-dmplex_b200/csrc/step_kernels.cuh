@@ -25,6 +25,8 @@
 #include <cfloat>
 #include <cstdint>
 
+#include "rn_div.h"
+
 namespace zsme {
 
 // ------------------------------------------------------------------ layout
@@ -233,10 +235,7 @@ __device__ __forceinline__ void cell_slots_gradient(const MeshDev& m, const Opts
             }
         }
         const double v = m.vol[c];
-        if (v > 1e-15) {
-#pragma unroll
-            for (int i = 0; i < NQ * DIM; ++i) g[i] /= v;
-        }
+        if (v > 1e-15) divide_all(g, v);
     }
 }
 
@@ -574,10 +573,7 @@ __global__ void __launch_bounds__(128, MINB) prep_lean_kernel(MeshDev m, Opts o,
             }
         }
         const double v = m.vol[c];
-        if (v > 1e-15) {
-#pragma unroll
-            for (int i = 0; i < NQ * DIM; ++i) g[i] /= v;
-        }
+        if (v > 1e-15) divide_all(g, v);
     }
     // pass 1: each face's alpha = min over components of min(vacuum, tvd)
     double al[KM];
@@ -784,10 +780,7 @@ __global__ void __launch_bounds__(128, MINB) prep_split_kernel(MeshDev m, Opts o
                 }
             }
             const double v = m.vol[c];
-            if (v > 1e-15) {
-#pragma unroll
-                for (int i = 0; i < NC * DIM; ++i) g[i] /= v;
-            }
+            if (v > 1e-15) divide_all(g, v);
         }
         // pass 1: this part's alpha per face = min over its components
         if (o.limiter) {
