@@ -134,7 +134,7 @@ __device__ __forceinline__ int imex_solve_fast(double hg, const double* z, doubl
         for (int e = 0; e < NQ * NA; ++e) need |= dSdA[e] != 0.0;
 #pragma unroll
         for (int i = 0; i < NQ; ++i) need |= !isfinite(ys[i]);
-        if (need || !newton_fast<M>(hg, y, res, dSdQ)) return -1;
+        if (need || !newton_fast<M>(hg, y, res, ys, a, p, dSdQ)) return -1;
     }
     return iter >= 15 ? 1 : 0;
 }

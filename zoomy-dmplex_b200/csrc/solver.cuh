@@ -455,11 +455,11 @@ class Solver final : public SolverBase {
         ZSME_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
         ZSME_CUDA(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device_));
         LaunchConfig lc{128, 128, 128, 128};
-        // finalize's register cap: us per launch on a B200 uncapped and capped, level 4
-        // at 2.0 M cells 459 and 424 (3 blocks of 128; 4: 438), level 2 at 977 k cells
-        // 157 and 119 (4: 124), level 1 at 498 k cells 45.2 and 39.7 (4; 3: 45.2);
-        // level 0 needs no more registers than any cap leaves
-        lc.finalize_occ = NQ >= 8 ? 3 : (NQ >= 6 ? 4 : 1);
+        // finalize's register cap: us per launch on a B200 uncapped, 3 and 4 blocks of
+        // 128 per SM: level 4 at 231 k cells 56.1, 47.2, 48.9; level 2 at 977 k cells
+        // 152.6, 114.8, 110.3; level 1 at 498 k cells 45.2, 45.2, 39.7; level 0 needs
+        // no more registers than any cap leaves
+        lc.finalize_occ = NQ >= 10 ? 3 : (NQ >= 6 ? 4 : 1);
         // the separate face kernel's (adjoint replays): level 4, us per launch at 2.0 M
         // cells, 3 blocks per SM 350, uncapped 407; level 2 the same within 2 %
         lc.face_occ = NQ >= 10 ? 3 : 4;

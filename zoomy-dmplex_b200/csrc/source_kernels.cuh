@@ -38,8 +38,9 @@ struct SmeLayout {
 // One Newton update on the fast path; returns 1 if q was updated, 0 to fall
 // back to the generic path (structure not met, or a singular / non-finite
 // pivot, which the generic path then handles exactly as the reference).
-template <class M>
-__device__ __forceinline__ int newton_fast(double dtl, double* q, const double* res,
+// UNSWAPPED: by gepp_unswapped; returns -1, q unchanged, for an odd cell.
+template <class M, bool UNSWAPPED>
+__device__ __forceinline__ int newton_block(double dtl, double* q, const double* res,
                                            const SimpleArray<double, M::n_dof_q * M::n_dof_q>& S) {
     using L = SmeLayout<M>;
     constexpr int NQ = L::NQ, NM = L::NM, NB = L::NB, DIM = L::DIM;
@@ -66,7 +67,7 @@ __device__ __forceinline__ int newton_fast(double dtl, double* q, const double* 
         }
         if (!fast) return 0;
         double xm[NB];
-        bool ok = true;
+        bool ok = true, odd = false;
         if (DIM == 1 || split) {
 #pragma unroll
             for (int d = 0; d < DIM; ++d) {
@@ -81,7 +82,8 @@ __device__ __forceinline__ int newton_fast(double dtl, double* q, const double* 
                     }
                     b[a] = -res[2 + d * NM + a];
                 }
-                ok &= gepp_regs<NM>(A, b, x);
+                if constexpr (UNSWAPPED) ok &= gepp_unswapped<NM>(A, b, x, odd);
+                else ok &= gepp_regs<NM>(A, b, x);
 #pragma unroll
                 for (int a = 0; a < NM; ++a) xm[d * NM + a] = x[a];
             }
@@ -97,16 +99,44 @@ __device__ __forceinline__ int newton_fast(double dtl, double* q, const double* 
                     }
                     b[a] = -res[2 + a];
                 }
-                ok &= gepp_regs<NB>(A, b, x);
+                if constexpr (UNSWAPPED) ok &= gepp_unswapped<NB>(A, b, x, odd);
+                else ok &= gepp_regs<NB>(A, b, x);
 #pragma unroll
                 for (int a = 0; a < NB; ++a) xm[a] = x[a];
             }
         }
+        if (odd) return -1;
         if (!ok || !isfinite(dtl)) return 0;
 #pragma unroll
         for (int a = 0; a < NB; ++a) q[2 + a] += xm[a];
         return 1;
     }
+}
+// The update at the state qs with aux as, whose Jacobian is S.  Odd cells (none
+// in the benchmark flows; stiff slip friction swaps rows) evaluate the Jacobian
+// again, from values the compiler cannot recognise, so that S need not stay in
+// registers for them.
+template <class M>
+__device__ __forceinline__ int newton_fast(double dtl, double* q, const double* res, const double* qs,
+                                           const double* as, const double* p,
+                                           const SimpleArray<double, M::n_dof_q * M::n_dof_q>& S) {
+    constexpr int NQ = M::n_dof_q, NA = M::n_dof_qaux;
+    int rc = newton_block<M, true>(dtl, q, res, S);
+    if (rc < 0) {
+        double qv[NQ], av[NA];
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+            qv[i] = qs[i];
+            asm volatile("" : "+d"(qv[i]));
+        }
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            av[i] = as[i];
+            asm volatile("" : "+d"(av[i]));
+        }
+        rc = newton_block<M, false>(dtl, q, res, M::source_jacobian_wrt_variables(qv, av, p));
+    }
+    return rc;
 }
 
 // iters (optional): Newton updates applied (0 when the first residual is below
@@ -145,7 +175,7 @@ __device__ __forceinline__ int newton_cell(double dtl, double* q, double* aux, c
         for (int e = 0; e < NQ * NA; ++e) need |= (dSdA[e] != 0.0);
 #pragma unroll
         for (int i = 0; i < NQ; ++i) need |= !isfinite(q[i]);
-        if (!need && newton_fast<M>(dtl, q, res, dSdQ)) continue;
+        if (!need && newton_fast<M>(dtl, q, res, q, aux, p, dSdQ)) continue;
         if constexpr (!GENERIC) {
             return -1;
         } else {
