@@ -641,22 +641,22 @@ class Solver final : public SolverBase {
             ZSME_CUDA(cudaMemcpyAsync(tmp_a_.p, q, (size_t)NQ * cn * sizeof(double), cudaMemcpyHostToDevice, stream_));
             src = tmp_a_.p;
         }
-        aos_to_soa_kernel<<<blocks_for(cn, 128), 128, 0, stream_>>>(src, x_.p, old_of_new_.p, c0, cn, pm_.C, NQ);
+        load_state(inst, c0, cn, src, t);
         ZSME_CUDA(cudaGetLastError());
-        set_time_kernel<<<1, 1, 0, stream_>>>(t_.p + inst, t);
         rc = enqueue_loaded(inst, c0, cn);
         if (rc) return rc;
         ZSME_CUDA(cudaStreamSynchronize(stream_));
         return ZSME_OK;
     }
-    // After a state (and its time) is in place: aux reset, constraints, then
+    void load_state(int inst, int c0, int cn, const double* aos, double t) {
+        load_state_kernel<<<blocks_for(std::max(cn, 8), 128), 128, 0, stream_>>>(
+            aos, x_.p, old_of_new_.p, c0, cn, pm_.C, NQ, aux_.p, NA, t_.p + inst, t, active_.p + inst,
+            inst == 0 ? iscal_.p : nullptr);
+    }
+    // After load_state: constraints, then
     // dt_start = max(ComputeTimeStep, min_dt) (MUSCLSolver.hpp:51-54, 103).
     int enqueue_loaded(int inst, int c0, int cn) {
         imp_have_prev_ = false;   // the implicit strategy restarts at BDF order 1
-        for (int k = 0; k < NA; ++k)
-            ZSME_CUDA(cudaMemsetAsync(aux_.p + (size_t)k * pm_.C + c0, 0, cn * sizeof(double), stream_));
-        ZSME_CUDA(cudaMemsetAsync(active_.p + inst, 0, sizeof(int), stream_));
-        if (inst == 0) ZSME_CUDA(cudaMemsetAsync(iscal_.p, 0, 8 * sizeof(int), stream_));
         StepDev sd = step_dev(nullptr);
         sd.active = nullptr;
         launch_derivative_aux(x_.p, nullptr);      // PostStep's UpdateState: the derivative aux first
@@ -738,10 +738,9 @@ class Solver final : public SolverBase {
         ZSME_CUDA(cudaMemcpyAsync(in_stage_[j].p, q, (size_t)NQ * C * sizeof(double), cudaMemcpyHostToDevice, h2d_));
         ZSME_CUDA(cudaEventRecord(ev_h2d_[j], h2d_));
         ZSME_CUDA(cudaStreamWaitEvent(stream_, ev_h2d_[j], 0));
-        aos_to_soa_kernel<<<blocks_for(C, 128), 128, 0, stream_>>>(in_stage_[j].p, x_.p, old_of_new_.p, 0, C, C, NQ);
+        load_state(0, 0, C, in_stage_[j].p, t);
         ZSME_CUDA(cudaGetLastError());
         ZSME_CUDA(cudaEventRecord(ev_in_used_[j], stream_));
-        set_time_kernel<<<1, 1, 0, stream_>>>(t_.p, t);
         return enqueue_loaded(0, 0, C);
     }
     int get_state_async(double* q) override {

@@ -1266,7 +1266,6 @@ static __global__ void end_step_kernel(StepDev sd, int i0, int ni, int mode, dou
 // AoS (caller order within an instance) <-> SoA (Hilbert order): cells
 // [c0, c0 + cn) of the SoA arrays (row stride C) are instance-local rows
 // old_of_new[c] of the AoS buffer.
-static __global__ void set_time_kernel(double* t, double v) { *t = v; }
 // q_aos[e] = state of caller cell cells[e] (ids outside [0, C) are skipped)
 static __global__ void get_cells_kernel(const double* __restrict__ soa, int C, int nq,
                                         const int* __restrict__ new_of_old, const int* __restrict__ cells, int n,
@@ -1309,6 +1308,26 @@ static __global__ void aos_to_soa_kernel(const double* __restrict__ aos, double*
     const int c = c0 + r;
     const int o = old_of_new[c];
     for (int i = 0; i < nq; ++i) soa[(size_t)i * C + c] = aos[(size_t)o * nq + i];
+}
+// A caller's state becomes instance inst's at time t, in one launch (a copy
+// kernel, two or three memsets and a time kernel before: 8 us of a 1 k-cell
+// pass): the components as aos_to_soa_kernel, the cells' aux variables zero,
+// the instance idle and, for instance 0, the counters iscal [0, 8) zero.
+static __global__ void load_state_kernel(const double* __restrict__ aos, double* __restrict__ soa,
+                                         const int* __restrict__ old_of_new, int c0, int cn, int C, int nq,
+                                         double* __restrict__ aux, int na, double* t, double t_value, int* active,
+                                         int* iscal) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r == 0) {
+        *t = t_value;
+        *active = 0;
+    }
+    if (r < 8 && iscal) iscal[r] = 0;
+    if (r >= cn) return;
+    const int c = c0 + r;
+    const int o = old_of_new[c];
+    for (int i = 0; i < nq; ++i) soa[(size_t)i * C + c] = aos[(size_t)o * nq + i];
+    for (int k = 0; k < na; ++k) aux[(size_t)k * C + c] = 0.0;
 }
 // Blocks of 128 cells through shared memory ([nq][129] doubles): the component
 // rows are read coalesced and a cell's components written next to one another,
