@@ -11,6 +11,7 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "model_prelude.h"
@@ -115,6 +116,7 @@ class Solver final : public SolverBase {
     DevBuf<int> st_ext_cell_, st_gho_cell_, st_gho_face_;
     DevBuf<unsigned> st_loc_;
     DevBuf<double> st_geo_;
+    int st_limit_ = 0, tile_limit_ = 0;   // the shared-memory limits that are set
     int st_built_ = 0, st_entries_ = 0, st_fst_ = 0, st_cst_ = 0;
     bool st_fits_ = false;
     bool ready_ = false;          // init done: mesh on the device
@@ -257,6 +259,36 @@ class Solver final : public SolverBase {
     // (Re)builds the tiles for lc_.tile_faces; outside any stream capture
     // (set-up and zsme_set_launch only).
     int ensure_tiles() {
+        const int rc = build_tile_tables();
+        return rc || lc_.tile_faces <= 0 ? rc : tile_limits();
+    }
+    // Dynamic shared memory of the kernel this launch shape runs, and of no other: each
+    // call loads the kernel's code (all twelve kernels cost a small handle 2 ms of set-up).
+    // A limit of the kernel, shared by every handle: always the largest.
+    int tile_limits() {
+        if (use_stage()) {
+            const int P = stage_parts(), bytes = (int)kMaxStageSmem;
+            if (st_limit_ == P) return ZSME_OK;
+            auto set = [&](auto k) {
+                constexpr int KM = decltype(k)::value;
+                if (well_balanced()) return stage_smem_limit<KM, 1, true>(bytes);
+                return P == 4 ? stage_smem_limit<KM, 4>(bytes)
+                              : (P == 2 ? stage_smem_limit<KM, 2>(bytes) : stage_smem_limit<KM, 1>(bytes));
+            };
+            ZSME_CUDA(pm_.K == 3 ? set(std::integral_constant<int, 3>()) : set(std::integral_constant<int, 4>()));
+            st_limit_ = P;
+            return ZSME_OK;
+        }
+        if (tile_limit_) return ZSME_OK;
+        const int smem = (int)kMaxTileSmem;
+        ZSME_CUDA(cudaFuncSetAttribute(flux_tile_kernel<M, N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        ZSME_CUDA(cudaFuncSetAttribute(flux_tile_kernel<M, N, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        ZSME_CUDA(cudaFuncSetAttribute(flux_tile_kernel<M, N, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        ZSME_CUDA(cudaFuncSetAttribute(flux_tile_kernel<M, N, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        tile_limit_ = 1;
+        return ZSME_OK;
+    }
+    int build_tile_tables() {
         if (lc_.tile_faces <= 0 || (tile_built_ == lc_.tile_faces && (st_built_ == lc_.tile_faces || !wants_stage())))
             return ZSME_OK;
         FaceTiles t;
@@ -272,12 +304,6 @@ class Solver final : public SolverBase {
         ZSME_CUDA(tile_ord_lf_.upload(t.ord_lf, stream_));
         tile_n_ = t.n;
         tile_stride_ = t.max_faces;
-        // a limit of the kernel, shared by every handle: always the largest
-        const int smem = (int)kMaxTileSmem;
-        ZSME_CUDA(cudaFuncSetAttribute(flux_tile_kernel<M, N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        ZSME_CUDA(cudaFuncSetAttribute(flux_tile_kernel<M, N, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        ZSME_CUDA(cudaFuncSetAttribute(flux_tile_kernel<M, N, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        ZSME_CUDA(cudaFuncSetAttribute(flux_tile_kernel<M, N, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         tile_built_ = lc_.tile_faces;
         return ZSME_OK;
     }
@@ -388,12 +414,6 @@ class Solver final : public SolverBase {
                                                        st_.gradient == ZSME_GRADIENT_LSQ, st_geo_.p);
         ZSME_CUDA(cudaGetLastError());
         ZSME_CUDA(cudaStreamSynchronize(stream_));   // a chained launch reads it without waiting for the stream
-        const int bytes = (int)kMaxStageSmem;   // a limit of the kernel, shared by every handle
-#define ZSME_STAGE_ATTR(...)                                                                                       \
-    ZSME_CUDA((stage_smem_limit<3, __VA_ARGS__>(bytes)));                                                           \
-    ZSME_CUDA((stage_smem_limit<4, __VA_ARGS__>(bytes)));
-        ZSME_STAGE_ATTR(1) ZSME_STAGE_ATTR(2) ZSME_STAGE_ATTR(4) ZSME_STAGE_ATTR(1, true)
-#undef ZSME_STAGE_ATTR
         return ZSME_OK;
     }
     int stage_row(int parts, int n) const {
