@@ -94,22 +94,32 @@ def peaks():
     return 6650.0, "fallback"
 
 
-def algorithmic_bytes(kind, C, F, nq, na, K, stages, fused=False):
+def flux_form(launch):
+    """What the kernel kind "flux" is under a launch configuration: the whole
+    stage ("stage"), face + gather ("tile") or the face kernel alone ("face")."""
+    if launch["tile_faces"] <= 0:
+        return "face"
+    return "stage" if launch["fuse_final"] else "tile"
+
+
+def algorithmic_bytes(kind, C, F, nq, na, K, stages, form="face"):
     """Compulsory HBM bytes of one launch of each kernel when every array it
     touches is read or written exactly once (neighbour re-reads are free).
-    fused: "flux" is the fused face + gather tile kernel (face states,
-    geometry and support in, the stage's state in and out; no face
-    contributions in device memory)."""
+    form: what "flux" is (flux_form).  The tile kernel takes face states,
+    geometry and support in and the stage's state in and out; the whole-stage
+    kernel the state, per cell its connectivity, face geometry and volume, per
+    face normal, area and support, and the next state out."""
     d = 2
+    state_passes = (2 * (stages - 1) + 3) / stages          # FIRST/MID: in+out, FINAL: in+base+out
+    if kind == "flux" and form == "stage":
+        return C * (8 * nq * state_passes + 8 * K + 16 * d * K + 16) + F * (8 * (d + 1) + 12)
     if kind == "prep":      # state + aux + slot tables in, two face states per face out
         return C * (8 * nq + 8 * na + 12 * K + 16 * d * K) + F * 16 * nq
-    if kind == "flux" and fused:
-        state_passes = (2 * (stages - 1) + 3) / stages      # FIRST/MID: in+out (+ clamped copy), FINAL: in+base+out
+    if kind == "flux" and form == "tile":                   # FIRST/MID write the clamped copy too
         return F * (16 * nq + 8 * (2 * d + 1) + 12) + C * (8 * na + 4 * K + 8 + 8 * nq * state_passes)
     if kind == "flux":      # face kernel: two face states + geometry + support in, 3 NQ contributions out
         return F * (16 * nq + 8 * (2 * d + 1) + 12 + 24 * nq) + C * 8 * na
     if kind == "gather":    # 3 NQ contributions per face in, state in/out
-        state_passes = (2 * (stages - 1) + 3) / stages      # FIRST/MID: in+out, FINAL: in+base+out
         return F * 24 * nq + C * (12 * K + 4 + 8 + 8 * nq * state_passes)
     if kind == "finalize":
         return C * (16 * nq + 16 * na + 8)
@@ -124,19 +134,15 @@ def step_bytes_fused(nq):
 
 
 # DRAM bytes (read + write) per cell of one launch, from the ncu captures of
-# profiles/sme2d_l4_kernels_900.md (900x900 grid, 1,616,402 cells; mean of
-# two launches) in the launch configuration the autotuner picks at level 4:
-# separate face and gather kernels, the face-state kernel split over four
-# threads per cell, the last stage's gather inside finalize (register cap 4).
-# The streams scale with the cell count, so a 1400x1400 launch moves these
-# figures times its cells.
+# profiles/sme2d_l4_stage_900.md (900x900 grid, 1,616,402 cells; the stage
+# kernel's two launches and finalize of one step) in the launch configuration a
+# level-4 handle of that size starts with.  The streams scale with the cell
+# count, so a 1400x1400 launch moves these figures times its cells.
 NCU_DRAM_BYTES_PER_CELL = {
-    "sme2d_l4/prep": (436.6 + 425.4) * 1e6 / 1616402,
-    "sme2d_l4/flux": (544.7 + 652.4) * 1e6 / 1616402,
-    "sme2d_l4/gather": (1143.8 + 282.5) * 1e6 / 1616402,
-    "sme2d_l4/finalize+gather": (1125.9 + 422.2) * 1e6 / 1616402,
+    "sme2d_l4/flux": (520.6 + 177.9 + 675.5 + 178.3) / 2 * 1e6 / 1616402,
+    "sme2d_l4/finalize": (181.1 + 116.2) * 1e6 / 1616402,
 }
-NCU_LAUNCH = {"tile_faces": 0, "fuse_final": 1, "prep_lean": 4}
+NCU_LAUNCH = {"tile_faces": 256, "fuse_final": 1}
 
 
 def traffic_per_cell_step(model, launch, stages):
@@ -146,7 +152,7 @@ def traffic_per_cell_step(model, launch, stages):
     if model != "sme2d_l4" or any(launch.get(k) != v for k, v in NCU_LAUNCH.items()) or stages != 2:
         return None
     t = NCU_DRAM_BYTES_PER_CELL
-    return 2 * t["sme2d_l4/prep"] + 2 * t["sme2d_l4/flux"] + t["sme2d_l4/gather"] + t["sme2d_l4/finalize+gather"]
+    return 2 * t["sme2d_l4/flux"] + t["sme2d_l4/finalize"]
 
 
 # Algorithmic FP64 operations per unit of each kernel: +, -, *, /, sqrt,
@@ -165,15 +171,15 @@ FP64_FLOPS = {
 }
 
 
-def fp64_flops(kind, model, C, F, stages, fused=False):
+def fp64_flops(kind, model, C, F, stages, form="face"):
     """Algorithmic FP64 operations of one launch of a step kernel (None
-    where the table has no figure); fused: "flux" is the fused face + gather
-    tile kernel, which does both kernels' work."""
+    where the table has no figure); form: what "flux" is (flux_form), with the
+    work of the kernels it stands for."""
     t = FP64_FLOPS.get(model, {})
     if kind not in t:
         return None
-    if kind == "flux" and fused:
-        return t["flux"] * F + t["gather"] * C
+    if kind == "flux" and form != "face":
+        return t["flux"] * F + (t["gather"] + (t["prep"] if form == "stage" else 0.0)) * C
     return t[kind] * (F if kind == "flux" else C)
 
 
@@ -874,7 +880,7 @@ def main():
     from zoomy_dmplex_b200.solver import get_launch
 
     launch_cfg = get_launch(g.h)
-    fused = launch_cfg["tile_faces"] > 0
+    fused = flux_form(launch_cfg)
     dom = max((k for k in prof if prof[k][1] > 0), key=lambda k: prof[k][0])
     dom_ms = prof[dom][0] / prof[dom][1]
     alg = algorithmic_bytes(dom, C, F, nq, na, case.mesh.max_faces, case.settings.ssp_stages, fused)
@@ -916,12 +922,14 @@ def main():
             if fl is not None:
                 v["fp64_tflops"] = fl / (v["ms_per_launch"] / 1e3) / 1e12
         fk = max((k for k in kernel_share if "fp64_tflops" in kernel_share[k]),
-                 key=lambda k: kernel_share[k]["fp64_tflops"])
+                 key=lambda k: kernel_share[k]["share"])
         fl = fp64_flops(fk, case.model, C, F, s_, fused)
         ach = kernel_share[fk]["fp64_tflops"]
         roofline_fp64 = {"bound": "fp64", "kernel": fk, "achieved": ach, "peak": peak_tf, "unit": "TFLOP/s",
                          "frac": ach / peak_tf, "frac_of_unfused": ach / (peak_tf / 2),
                          "flops_per_launch": fl,
+                         "flops_basis": "operations of the plain scheme (oracle count); finalize leaves out those on "
+                                        "structural zeros, so its rate is no measure of the pipe",
                          "peak_source": "measured on this GPU: zsme_fp64_fma_peak (FMA chains, 2 flops per FMA)"}
         fc = fp64_flops_per_cell_step(case.model, C, F, s_)
         ach_s = fc * C / (step_ms / 1e3) / 1e12
