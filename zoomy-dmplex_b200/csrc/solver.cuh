@@ -262,8 +262,8 @@ class Solver final : public SolverBase {
         const int rc = build_tile_tables();
         return rc || lc_.tile_faces <= 0 ? rc : tile_limits();
     }
-    // Dynamic shared memory of the kernel this launch shape runs, and of no other: each
-    // call loads the kernel's code (all twelve kernels cost a small handle 2 ms of set-up).
+    // Dynamic shared memory of the kernel this launch shape runs, and of no other: a
+    // limit may load the kernel's code. What it saves is within the noise of set-up times.
     // A limit of the kernel, shared by every handle: always the largest.
     int tile_limits() {
         if (use_stage()) {
