@@ -957,7 +957,7 @@ class Solver final : public SolverBase {
                                                                                    active, aux_.p, params_.p, xl_out);
         mark(ZSME_KERNEL_GATHER, false);
     }
-    // fg: the last SSP stage's gather, fused into the finalize kernel (or nullptr)
+    // fg: the last SSP stage's gather, fused into the finalize kernel (or nullptr); with or without the source
     // x_src: the state to finalize where it is not x_ itself (the last stage's output buffer);
     // chained: the step's tail with it (step_tail_kernel), sd.n_fallback being zero
     void finalize_range(int c0, int cn, const StepDev& sd, const double* dt_src, int flags,
@@ -971,10 +971,7 @@ class Solver final : public SolverBase {
         const bool early = tile_n_ <= 4 * kStageBlocks * sm_count_;
         if ((flags & FIN_SOURCE) && !chained) cudaMemsetAsync(sd.n_fallback, 0, sizeof(int), stream_);
         mark(ZSME_KERNEL_FINALIZE, true);
-        if (!(flags & FIN_SOURCE)) {
-            launch_chained(early, finalize_kernel<M, N, 4, false, false>, gb, lc_.finalize, 0, md_, c0, cn, x_src, x_.p,
-                           aux_.p, params_.p, sd, dt_src, flags, FinalGather{});
-        } else if (fg) {
+        if (fg) {
             switch (lc_.finalize_occ) {
 #define ZSME_FING(OCC)                                                                                           \
     case OCC:                                                                                                    \
@@ -985,6 +982,9 @@ class Solver final : public SolverBase {
                 default: ZSME_FING(1)
 #undef ZSME_FING
             }
+        } else if (!(flags & FIN_SOURCE)) {
+            launch_chained(early, finalize_kernel<M, N, 4, false, false>, gb, lc_.finalize, 0, md_, c0, cn, x_src, x_.p,
+                           aux_.p, params_.p, sd, dt_src, flags, FinalGather{});
         } else {
             switch (lc_.finalize_occ) {
 #define ZSME_FIN(OCC)                                                                                            \
