@@ -40,9 +40,9 @@ struct FaceGeom {
 
 template <class M, class N>
 __device__ __forceinline__ bool face_contrib(const MeshDev& m, const FaceGeom& fg, const double* fs, size_t fstride,
-                                             const double* __restrict__ aux, const double* __restrict__ params,
+                                             const double* aux, const double* __restrict__ params,
                                              double t_host, const double* t_dev, double stage_frac,
-                                             const double* __restrict__ dt_step, const int* __restrict__ active,
+                                             const double* dt_step, const int* active,
                                              double* out, size_t ostride) {
     constexpr int NQ = M::n_dof_q, NA = M::n_dof_qaux;
     const int F = m.F, C = m.C;

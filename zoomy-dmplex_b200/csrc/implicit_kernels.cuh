@@ -34,9 +34,8 @@ struct BdfTerms {
 };
 
 template <class M>
-__device__ __forceinline__ void imp_residual_cell(const MeshDev& m, int c, const double* __restrict__ y,
-                                                  const double* __restrict__ aux, const double* __restrict__ params,
-                                                  const double* __restrict__ R, const BdfTerms& b,
+__device__ __forceinline__ void imp_residual_cell(const MeshDev& m, int c, const double* y, const double* aux,
+                                                  const double* __restrict__ params, const double* R, const BdfTerms& b,
                                                   double (&f)[M::n_dof_q]) {
     constexpr int NQ = M::n_dof_q, NA = M::n_dof_qaux;
     const int C = m.C;
@@ -427,11 +426,9 @@ __global__ void __launch_bounds__(128) imp_update_state_kernel(MeshDev m, const 
 // quotient (zero when hv is zero) and the block solve of a cell in one pass
 // (29 us as three kernels for 29 k level-2 cells).
 template <class M>
-__global__ void __launch_bounds__(128) imp_apply_kernel(MeshDev m, const double* __restrict__ y,
-                                                        const double* __restrict__ aux,
-                                                        const double* __restrict__ params,
-                                                        const double* __restrict__ R, BdfTerms b,
-                                                        const double* __restrict__ F0, const double* __restrict__ hv,
+__global__ void __launch_bounds__(128) imp_apply_kernel(MeshDev m, const double* y, const double* aux,
+                                                        const double* __restrict__ params, const double* R, BdfTerms b,
+                                                        const double* F0, const double* hv,
                                                         const double* __restrict__ lu, const int* __restrict__ piv,
                                                         const double* __restrict__ rdiag, double* __restrict__ out) {
     constexpr int NQ = M::n_dof_q;
@@ -453,8 +450,8 @@ __global__ void __launch_bounds__(128) imp_apply_kernel(MeshDev m, const double*
 // ------------------------------------------------------------ vector kernels
 static __global__ void imp_sqrt_kernel(const double* __restrict__ in, double* __restrict__ out) { *out = sqrt(*in); }
 // out = 1.0 x + hv v, hv a device scalar
-static __global__ void imp_perturb_kernel(long long n, const double* __restrict__ x, const double* __restrict__ v,
-                                          const double* __restrict__ hv, double* __restrict__ out) {
+static __global__ void imp_perturb_kernel(long long n, const double* x, const double* v, const double* hv,
+                                          double* __restrict__ out) {
     grid_release();
     grid_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -539,8 +536,8 @@ __device__ __forceinline__ void imp_finish_dots(const double (&s)[NK], int k0, i
 }
 // out[k] = V_k . w, k < nk (V_k = V + k ld): NK vectors per block row
 template <int NK>
-__global__ void __launch_bounds__(256) imp_multi_dot_kernel(long long n, int nk, const double* __restrict__ V,
-                                                            long long ld, const double* __restrict__ w, DotSink d) {
+__global__ void __launch_bounds__(256) imp_multi_dot_kernel(long long n, int nk, const double* V, long long ld,
+                                                            const double* w, DotSink d) {
     grid_release();
     grid_wait();
     const int k0 = blockIdx.y * NK;
@@ -562,9 +559,8 @@ __global__ void __launch_bounds__(256) imp_multi_dot_kernel(long long n, int nk,
 }
 // w -= sum_k h_k V_k (classical Gram-Schmidt projection, h on the device) and
 // out[0] = w.w; four elements' chains run side by side
-static __global__ void __launch_bounds__(256) imp_project_kernel(long long n, int nk, const double* __restrict__ V,
-                                                                 long long ld, const double* __restrict__ h,
-                                                                 double* __restrict__ w, DotSink d) {
+static __global__ void __launch_bounds__(256) imp_project_kernel(long long n, int nk, const double* V, long long ld,
+                                                                 const double* h, double* __restrict__ w, DotSink d) {
     grid_release();
     grid_wait();
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -591,8 +587,7 @@ static __global__ void __launch_bounds__(256) imp_project_kernel(long long n, in
     imp_finish_dots<1>(sum, 0, 1, 0, d);
 }
 // v = (1.0 / sqrt(ww)) w where ww = w.w > 0 (the next Arnoldi vector) and out[0] = v.v
-static __global__ void __launch_bounds__(256) imp_normalize_kernel(long long n, const double* __restrict__ ww,
-                                                                   const double* __restrict__ w,
+static __global__ void __launch_bounds__(256) imp_normalize_kernel(long long n, const double* ww, const double* w,
                                                                    double* __restrict__ v, DotSink d) {
     grid_release();
     grid_wait();

@@ -239,7 +239,7 @@ enum FinalizeFlags {
 template <class M, class N, bool GENERIC, bool GATHER = false, bool SOURCE = true>
 __device__ __forceinline__ int finalize_cell(const MeshDev& m, int c, int I, const double* x_src, double* x,
                                              double* __restrict__ aux, const double* p, const StepDev& sd,
-                                             const double* __restrict__ dt_src, int flags, double& ratio,
+                                             const double* dt_src, int flags, double& ratio,
                                              const FinalGather* fg = nullptr) {
     constexpr int NQ = M::n_dof_q, NA = M::n_dof_qaux, DIM = M::dimension;
     const int C = m.C;
@@ -359,7 +359,7 @@ __device__ __forceinline__ void block_ratio_min(const StepDev& sd, int I, double
 template <class M, class N, int MINB, bool GATHER = false, bool SOURCE = true>
 __global__ void __launch_bounds__(128, MINB) finalize_kernel(MeshDev m, int c0, int cn, const double* x_src,
                                                        double* x, double* __restrict__ aux,
-                                                       const double* __restrict__ params, StepDev sd, const double* __restrict__ dt_src, int flags,
+                                                       const double* __restrict__ params, StepDev sd, const double* dt_src, int flags,
                                                        FinalGather fg = FinalGather{}) {
     constexpr int NQ = M::n_dof_q;
     grid_release();
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(128, MINB) finalize_kernel(MeshDev m, int c0, 
 template <class M, class N>
 __device__ __forceinline__ void finalize_deferred(const MeshDev& m, const double* x_src, double* x,
                                                   double* __restrict__ aux, const double* __restrict__ params,
-                                                  const StepDev& sd, const double* __restrict__ dt_src, int flags,
+                                                  const StepDev& sd, const double* dt_src, int flags,
                                                   int n) {
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(&sd.diag[6], n);
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
@@ -406,7 +406,7 @@ template <class M, class N>
 __global__ void __launch_bounds__(64) finalize_fallback_kernel(MeshDev m, const double* x_src, double* x,
                                                                double* __restrict__ aux,
                                                                const double* __restrict__ params, StepDev sd,
-                                                               const double* __restrict__ dt_src, int flags) {
+                                                               const double* dt_src, int flags) {
     finalize_deferred<M, N>(m, x_src, x, aux, params, sd, dt_src, flags, *sd.n_fallback);
 }
 
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(64) finalize_fallback_kernel(MeshDev m, const 
 template <class M, class N>
 __global__ void __launch_bounds__(64) step_tail_kernel(MeshDev m, const double* x_src, double* x,
                                                        double* __restrict__ aux, const double* __restrict__ params,
-                                                       StepDev sd, const double* __restrict__ dt_src, int flags) {
+                                                       StepDev sd, const double* dt_src, int flags) {
     grid_release();
     grid_wait();
     const int n = *sd.n_fallback;

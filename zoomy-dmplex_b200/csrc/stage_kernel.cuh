@@ -112,12 +112,10 @@ static __global__ void __launch_bounds__(128) stage_entries_kernel(MeshDev m, co
 template <class M, class N, int P, int KM, int THREADS, int MINB, bool WB = false>
 __global__ void __launch_bounds__(THREADS, MINB) stage_kernel(MeshDev m, Opts o, StageTilesDev tl,
                                                               StageWeights sc, StagePositivity pos,
-                                                              const double* __restrict__ x_in,
-                                                              const double* __restrict__ aux,
+                                                              const double* x_in, const double* aux,
                                                               const double* __restrict__ params, double t_host,
                                                               const double* t_dev, double stage_frac,
-                                                              const double* __restrict__ dt_step,
-                                                              const int* __restrict__ active, int mode,
+                                                              const double* dt_step, const int* active, int mode,
                                                               double* x_out, double* base) {
     constexpr int NQ = M::n_dof_q, NA = M::n_dof_qaux, DIM = M::dimension;
     constexpr int NC = StageShape<NQ, P>::NC;

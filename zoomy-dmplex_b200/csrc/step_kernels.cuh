@@ -78,7 +78,11 @@ struct StepDev {
 // start while its predecessor in the stream still runs; grid_wait() returns
 // once the predecessor is complete and its writes are visible (at once in a
 // plain launch), so everything before it may only touch what no kernel of the
-// stream writes (the mesh and its tiles).  grid_release() lets the successor
+// stream writes (the mesh and its tiles).  What a running predecessor may still
+// write is read through pointers without const __restrict__, which would state
+// that it stays as it is for the whole kernel (and let the compiler load it
+// through the non-coherent path); a restricted pointer that the kernel itself
+// writes through is no such statement.  grid_release() lets the successor
 // start as soon as every block of this grid has started.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -127,7 +131,7 @@ __device__ __forceinline__ void clamp_q(double* q, const double* a, const double
 }
 
 template <int NQ>
-__device__ __forceinline__ void load_q(const double* __restrict__ w, int C, int c, double* q) {
+__device__ __forceinline__ void load_q(const double* w, int C, int c, double* q) {
 #pragma unroll
     for (int i = 0; i < NQ; ++i) q[i] = w[(size_t)i * C + c];
 }
