@@ -636,8 +636,8 @@ __global__ void __launch_bounds__(THREADS, MINB) stage_kernel(MeshDev m, Opts o,
 
     // ---- sums, / volume and the stage combination (gather_kernel, stage_update),
     // NCG components per thread; consecutive threads, consecutive cells
-    constexpr int NCG = NQ % 4 == 0 ? 4 : (NQ % 3 == 0 ? 3 : 2), G = (NQ + NCG - 1) / NCG;
-    static_assert(G * NCG == NQ, "the parts cover the components");
+    // (the largest of 4, 3, 2, 1 that divides them: a 5-component plugin takes one each)
+    constexpr int NCG = NQ % 4 == 0 ? 4 : (NQ % 3 == 0 ? 3 : (NQ % 2 == 0 ? 2 : 1)), G = NQ / NCG;
     for (int task = tid; task < n * G; task += nt) {
         const int part = task / n, l = task - part * n;
         const int i0 = part * NCG, c = tile.c0 + l;
