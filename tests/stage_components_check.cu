@@ -116,7 +116,9 @@ template <int KM>
 static void compare_all(const Tables& t, const std::vector<double>& q4) {
     const std::vector<double> want = rhs<4, 1, KM>(t, q4);
     compare_parts<5, KM>(t, q4, want);
-    compare_parts<7, KM>(t, q4, want);
+    compare_parts<9, KM>(t, q4, want);
+    compare_parts<13, KM>(t, q4, want);
+    compare_parts<14, KM>(t, q4, want);
 }
 
 int main(int argc, char** argv) {

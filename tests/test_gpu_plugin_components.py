@@ -1,7 +1,8 @@
 """The whole-stage kernel for component counts that no shipped plugin has (a
-1-D level-2 plugin has 5, level 4 has 7): odd ones, whose sums one thread forms
-component by component.  It compiles (nvcc, no GPU needed) and, on a GPU, gives
-every component the values it has in a four-component plugin, bit for bit."""
+1-D level-2 plugin has 5, level 6 has 9): odd ones, whose sums one thread forms
+component by component, and ones that the threads of a cell do not share
+evenly.  It compiles (nvcc, no GPU needed) and, on a GPU, gives every component
+the values it has in a four-component plugin, bit for bit."""
 import os
 import shutil
 import subprocess
@@ -45,5 +46,5 @@ def test_components_equal_the_four_component_plugin(program, tmp_path, mesh):
             f.write(a[k].tobytes())
     r = subprocess.run([program, path], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
-    # both gradients, three thread counts, 5 + 7 components
-    assert r.stdout.split()[-4:] == ["checked", str(2 * 3 * 12), "wrong", "0"]
+    # both gradients, three thread counts, 5 + 9 + 13 + 14 components
+    assert r.stdout.split()[-4:] == ["checked", str(2 * 3 * 41), "wrong", "0"]

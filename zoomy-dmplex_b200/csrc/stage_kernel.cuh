@@ -246,8 +246,10 @@ __global__ void __launch_bounds__(THREADS, MINB) stage_kernel(MeshDev m, Opts o,
         }
         const RnDivisor by_vol(vol, rvol);
         const bool divide = !lsq && vol > 1e-15;
-        // a part beyond the last component repeats it: the same face states again
+        // a part beyond the last component repeats it: the same face states again,
+        // or none where its row still holds the increment that the state is formed of
         auto component = [&](int ii) { return NC * P == NQ ? i0 + ii : min(i0 + ii, NQ - 1); };
+        auto own = [&](int ii) { return KEEP || NC * P == NQ || i0 + ii < NQ; };
         auto load = [&](const double* from, int i, double& q, double (&v)[KM]) {
             q = from[i * cst + ent];
 #pragma unroll
@@ -513,7 +515,7 @@ __global__ void __launch_bounds__(THREADS, MINB) stage_kernel(MeshDev m, Opts o,
 #pragma unroll
                     for (int k = 0; k < KM; ++k) {
                         if constexpr (KEEP) inc[c4 + ii][k] = d[ii][k];
-                        else rows[component(c4 + ii) * fst + fso[k]] = d[ii][k];
+                        else if (own(c4 + ii)) rows[component(c4 + ii) * fst + fso[k]] = d[ii][k];
                     }
                 }
             }
@@ -599,7 +601,7 @@ __global__ void __launch_bounds__(THREADS, MINB) stage_kernel(MeshDev m, Opts o,
             }
 #pragma unroll
             for (int ii = 0; ii < CH; ++ii) {
-                if (c4 + ii >= NC) continue;
+                if (c4 + ii >= NC || !own(c4 + ii)) continue;
 #pragma unroll
                 for (int k = 0; k < KM; ++k) rows[component(c4 + ii) * fst + fso[k]] = q[ii] + al[k] * d[ii][k];
             }
