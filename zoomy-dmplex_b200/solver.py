@@ -370,17 +370,27 @@ LAUNCH_DEFAULTS = {"prep": 128, "face": 128, "gather": 128, "finalize": 128, "pr
                    "finalize_occ": 1, "tile_faces": 256, "fuse_final": 0, "prep_lean": 1}
 
 
+# which kernels run: whole stages, face + gather, or the separate ones
+KERNEL_KEYS = ("tile_faces", "fuse_final")
+
+
 def set_launch(h, cfg):
     """Launch configuration of a handle: dict with LAUNCH_KEYS (threads per
     block of each kernel, register caps as blocks per SM, tile_faces: 0 for
     the separate face and gather kernels, else the tile kernels' most faces
     per tile, fuse_final: with tiles the whole stage in one kernel, else the
     last stage's gather inside the finalize kernel, prep_lean: the lean
-    face-state kernel and its threads per cell); missing keys take
+    face-state kernel and its threads per cell).  A call that names neither
+    tile_faces nor fuse_final keeps the handle's kernels: these two, and
+    prep_lean unless named, stay as they are.  Other missing keys take
     LAUNCH_DEFAULTS.  A new handle has the configuration that get_launch
     returns, chosen by model and mesh size."""
     lib = native.load()
-    b = (ct.c_int32 * len(LAUNCH_KEYS))(*[int(cfg.get(k, LAUNCH_DEFAULTS[k])) for k in LAUNCH_KEYS])
+    missing = LAUNCH_DEFAULTS
+    if not any(k in cfg for k in KERNEL_KEYS):
+        own = get_launch(h)
+        missing = dict(missing, **{k: own[k] for k in KERNEL_KEYS + ("prep_lean",)})
+    b = (ct.c_int32 * len(LAUNCH_KEYS))(*[int(cfg.get(k, missing[k])) for k in LAUNCH_KEYS])
     native.check(lib.zsme_set_launch(h, b))
 
 
