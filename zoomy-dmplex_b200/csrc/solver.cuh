@@ -789,8 +789,7 @@ class Solver final : public SolverBase {
 
     // cells [c0, c0 + cn) of nv component rows into caller order
     void launch_to_aos(const double* soa, double* aos, int c0, int cn, int nv) {
-        soa_to_aos_kernel<<<blocks_for(cn, 128), 128, (size_t)129 * nv * sizeof(double), stream_>>>(
-            soa, aos, old_of_new_.p, c0, cn, pm_.C, nv);
+        launch_soa_to_aos(soa, aos, old_of_new_.p, c0, cn, pm_.C, nv, stream_);
     }
     int get_soa(int inst, const double* soa, int nv, double* out, bool device) {
         const int c0 = pm_.inst_cell_off[inst], cn = pm_.inst_cell_off[inst + 1] - c0;

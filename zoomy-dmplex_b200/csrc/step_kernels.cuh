@@ -1333,10 +1333,13 @@ static __global__ void load_state_kernel(const double* __restrict__ aos, double*
     for (int i = 0; i < nq; ++i) soa[(size_t)i * C + c] = aos[(size_t)o * nq + i];
     for (int k = 0; k < na; ++k) aux[(size_t)k * C + c] = 0.0;
 }
-// Blocks of 128 cells through shared memory ([nq][129] doubles): the component
-// rows are read coalesced and a cell's components written next to one another,
-// whole sectors of the caller's buffer (one thread per cell wrote one double
-// of a sector at a time: 221 us for 2.0 M cells of 12 components).
+// Blocks of 128 cells through shared memory ([rows][129] doubles, kAosRows
+// components at a time): the component rows are read coalesced and a cell's
+// components written next to one another, whole sectors of the caller's buffer
+// (one thread per cell wrote one double of a sector at a time: 221 us for 2.0 M
+// cells of 12 components).  The rows are bounded, so any number of components
+// fits the shared memory that a launch has without opting in.
+constexpr int kAosRows = 32;
 static __global__ void __launch_bounds__(128) soa_to_aos_kernel(const double* __restrict__ soa,
                                                                 double* __restrict__ aos,
                                                                 const int* __restrict__ old_of_new, int c0, int cn,
@@ -1344,15 +1347,24 @@ static __global__ void __launch_bounds__(128) soa_to_aos_kernel(const double* __
     extern __shared__ double tile[];
     __shared__ int old[128];
     const int r0 = blockIdx.x * 128, n = min(128, cn - r0), t = threadIdx.x;
-    if (t < n) {
-        old[t] = old_of_new[c0 + r0 + t];
-        for (int i = 0; i < nq; ++i) tile[i * 129 + t] = soa[(size_t)i * C + c0 + r0 + t];
+    if (t < n) old[t] = old_of_new[c0 + r0 + t];
+    for (int i0 = 0; i0 < nq; i0 += kAosRows) {
+        const int ni = min(kAosRows, nq - i0);
+        if (i0) __syncthreads();
+        if (t < n)
+            for (int i = 0; i < ni; ++i) tile[i * 129 + t] = soa[(size_t)(i0 + i) * C + c0 + r0 + t];
+        __syncthreads();
+        for (int e = t; e < n * ni; e += 128) {
+            const int l = e / ni, i = e - l * ni;
+            aos[(size_t)old[l] * nq + i0 + i] = tile[i * 129 + l];
+        }
     }
-    __syncthreads();
-    for (int e = t; e < n * nq; e += 128) {
-        const int l = e / nq, i = e - l * nq;
-        aos[(size_t)old[l] * nq + i] = tile[i * 129 + l];
-    }
+}
+static inline void launch_soa_to_aos(const double* soa, double* aos, const int* old_of_new, int c0, int cn, int C, int nq,
+                                     cudaStream_t stream) {
+    const int rows = nq < kAosRows ? nq : kAosRows;
+    soa_to_aos_kernel<<<(cn + 127) / 128, 128, (size_t)129 * rows * sizeof(double), stream>>>(soa, aos, old_of_new, c0,
+                                                                                             cn, C, nq);
 }
 
 }  // namespace zsme
