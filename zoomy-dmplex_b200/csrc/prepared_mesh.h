@@ -1,6 +1,7 @@
 // Model-independent host structures shared by the model translation units
 // and the C ABI layer: the device-ready mesh layout and the solver interface.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -44,6 +45,50 @@ struct LaunchConfig {
                                        // prep_split_kernel with 2..4 threads per cell; stage_kernel's
                                        // threads per cell: 1 (0, 1), 2, 4 (3, 4)
 };
+
+// Limits of the tile kernels: shared memory of the face + gather kernel (3 NQ
+// rows of the tile's faces) and of the whole-stage kernel, the latter's threads
+// and blocks per SM, which cap its registers: 128 per thread, 80 where the flux
+// needs no more (level 0: 380 against 436 us per step at 977 k cells; level 2
+// with 80: 468 against 414 at 498 k cells, spilling).
+constexpr size_t kMaxTileSmem = 200 * 1024, kMaxStageSmem = 227 * 1024;
+constexpr int kStageThreads = 256;
+constexpr int stage_blocks(int nq) { return nq >= 6 ? 2 : 3; }
+constexpr int kMinTileFaces = 64;   // zsme_set_launch takes 64..1024
+
+// The tiles a handle starts with.  With the whole-stage kernel: the
+// smallest (of at least 96 faces) that still fill the chip in one
+// wave, because within one wave a step's time is a tile's latency, and then
+// several threads per cell where a tile's cells leave threads of the block
+// idle; where one wave of the largest tiles does not cover the mesh, 256
+// faces, the least rim per cell that leaves stage_blocks blocks room in
+// shared memory.  us per step on a B200, level 4 at 15.8 k cells: 96 faces
+// and 2 threads per cell 45.1, 256 and 1 56.5; level 2 at 51.2 k cells: 320
+// faces 61.6, 256 71.5, 128 66.1; level 4 at 231 k cells: 256 342, 128 354,
+// 64 408.  A model of more than 53 components has no room for a tile of 64
+// faces and starts on the face + gather kernel: 256 faces or what fits, halved
+// while the mesh gives fewer than three tiles per SM.
+inline void default_tiles(LaunchConfig& lc, int nq, int faces, int sms) {
+    const int tf = std::min(256, (int)(kMaxTileSmem / (3 * nq * sizeof(double))));
+    const int blocks = stage_blocks(nq);
+    // a tile evaluates about 1 / 0.87 of the faces it owns; its rows take
+    // about 1.06 cells and 3 NQ doubles per face
+    const int room = (int)((kMaxStageSmem / blocks - 2048) / (8 * (1.06 * (nq + 4) + 3 * nq)));
+    const int largest = std::min(320, room / 32 * 32);
+    if (largest < kMinTileFaces) {
+        lc.fuse_final = 0;
+        lc.tile_faces = tf;
+        while (lc.tile_faces > kMinTileFaces && faces / lc.tile_faces < 3 * sms)
+            lc.tile_faces = std::max(kMinTileFaces, lc.tile_faces / 2);
+        return;
+    }
+    lc.fuse_final = 1;
+    const int wave = (int)(faces / (0.87 * blocks * sms));
+    const int one = std::max(96, (wave + 31) / 32 * 32);
+    lc.tile_faces = one <= largest ? one : std::min(tf, largest);
+    const int entries = (int)(0.85 * lc.tile_faces);   // cells with ring 1, triangles
+    lc.prep_lean = one > largest || 2 * entries > kStageThreads ? 1 : (4 * entries > kStageThreads ? 2 : 4);
+}
 
 // Tiles of the fused face + gather kernel.  A tile is a run of consecutive
 // cells; it evaluates the faces whose lowest cell lies in the tile (a

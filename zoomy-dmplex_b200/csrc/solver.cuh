@@ -254,8 +254,6 @@ class Solver final : public SolverBase {
         if (ready_) return ensure_tiles();
         return ZSME_OK;
     }
-    // Shared memory of one tile: 3 NQ rows of the tile's faces.
-    static constexpr size_t kMaxTileSmem = 200 * 1024;
     // (Re)builds the tiles for lc_.tile_faces; outside any stream capture
     // (set-up and zsme_set_launch only).
     int ensure_tiles() {
@@ -309,30 +307,6 @@ class Solver final : public SolverBase {
     }
     LaunchConfig launch() const override { return lc_; }
 
-    // The launch a handle starts with.  With the whole-stage kernel: the
-    // smallest tiles (of at least 96 faces) that still fill the chip in one
-    // wave, because within one wave a step's time is a tile's latency, and then
-    // several threads per cell where a tile's cells leave threads of the block
-    // idle; where one wave of the largest tiles does not cover the mesh, 256
-    // faces, the least rim per cell that leaves kStageBlocks blocks room in
-    // shared memory.  us per step on a B200, level 4 at 15.8 k cells: 96 faces
-    // and 2 threads per cell 45.1, 256 and 1 56.5; level 2 at 51.2 k cells: 320
-    // faces 61.6, 256 71.5, 128 66.1; level 4 at 231 k cells: 256 342, 128 354,
-    // 64 408.
-    void default_tiles(LaunchConfig& lc) const {
-        const int tf = std::min(256, (int)(kMaxTileSmem / (3 * NQ * sizeof(double))));
-        lc.fuse_final = 1;
-        // a tile evaluates about 1 / 0.87 of the faces it owns; its rows take
-        // about 1.06 cells and 3 NQ doubles per face
-        const int room = (int)((kMaxStageSmem / kStageBlocks - 2048) / (8 * (1.06 * (NQ + 4) + 3 * NQ)));
-        const int largest = std::min(320, room / 32 * 32);
-        const int wave = (int)(pm_.F / (0.87 * kStageBlocks * sm_count_));
-        const int one = std::max(96, (wave + 31) / 32 * 32);
-        lc.tile_faces = one <= largest ? one : std::min(tf, largest);
-        const int entries = (int)(0.85 * lc.tile_faces);   // cells with ring 1, triangles
-        lc.prep_lean = one > largest || 2 * entries > kStageThreads ? 1 : (4 * entries > kStageThreads ? 2 : 4);
-    }
-
     // A launch that may start while its predecessor drains (grid_wait in the
     // kernel); per-kernel timing keeps the kernels apart.
     template <class... KA, class... A>
@@ -351,12 +325,7 @@ class Solver final : public SolverBase {
     }
 
     // ------------------------------------------------------- whole-stage kernel
-    static constexpr int kStageThreads = 256;
-    static constexpr size_t kMaxStageSmem = 227 * 1024;
-        // blocks per SM, which caps the registers: 128 per thread, 80 where the flux
-    // needs no more (level 0: 380 against 436 us per step at 977 k cells; level 2
-    // with 80: 468 against 414 at 498 k cells, spilling)
-    static constexpr int kStageBlocks = NQ >= 6 ? 2 : 3;
+    static constexpr int kStageBlocks = stage_blocks(NQ);
     bool wants_stage() const {
         // MOOD at order 1 works on x_ between the stage and finalize
         return lc_.tile_faces > 0 && lc_.fuse_final &&
@@ -483,7 +452,7 @@ class Solver final : public SolverBase {
         // the separate face kernel's (adjoint replays): level 4, us per launch at 2.0 M
         // cells, 3 blocks per SM 350, uncapped 407; level 2 the same within 2 %
         lc.face_occ = NQ >= 10 ? 3 : 4;
-        default_tiles(lc);
+        default_tiles(lc, NQ, pm_.F, sm_count_);
         if (st_.block_size > 0) lc.prep = lc.face = lc.gather = st_.block_size;
         int rc = set_launch(lc);
         if (rc) return rc;
