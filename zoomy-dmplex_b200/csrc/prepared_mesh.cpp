@@ -33,9 +33,9 @@ uint64_t hilbert_d(uint32_t x, uint32_t y) {
     return d;
 }
 
-// Cholesky solve of the normal equations (Gradient.hpp:205-217).
-bool solve_spd(int n, std::vector<double>& a, std::vector<double>& b) {
-    std::vector<double> L(n * n, 0.0);
+// Cholesky solve of the n x n normal equations, n <= 2 (Gradient.hpp:205-217).
+bool solve_spd(int n, const double* a, double* b) {
+    double L[4] = {0.0, 0.0, 0.0, 0.0};
     for (int i = 0; i < n; i++) {
         for (int j = 0; j <= i; j++) {
             double sum = 0;
@@ -176,9 +176,11 @@ int prepare_mesh(const zsme_mesh& m, PreparedMesh& out, bool least_squares) {
         const int o = p.old_of_new[c];
         p.vol[c] = m.cell_volume[o];
         const double* xc = &m.cell_centroid[2 * o];
-        // neighbours in cone order for the least-squares system
-        std::vector<int> nb_slot, nb_cell;
-        std::vector<std::vector<double>> basis;
+        // neighbours in cone order for the least-squares system (at most one per
+        // slot; arrays, not vectors: the allocations were most of the set-up of a
+        // least-squares handle)
+        int nb = 0, nb_slot[4], nb_cell[4];
+        double basis[4][2];
         for (int k = 0; k < K; ++k) {
             const int f = m.cell_faces[(size_t)o * K + k];
             if (f < 0) continue;
@@ -205,22 +207,20 @@ int prepare_mesh(const zsme_mesh& m, PreparedMesh& out, bool least_squares) {
             const double dist = std::sqrt(d2);
             if (dist < p.rc[c]) p.rc[c] = dist;
             if (other >= 0 && least_squares) {
-                if (std::find(nb_cell.begin(), nb_cell.end(), other) != nb_cell.end()) continue;
-                nb_cell.push_back(other);
-                nb_slot.push_back(k);
-                std::vector<double> b;
-                for (int d = 0; d < D; ++d) b.push_back(m.cell_centroid[2 * other + d] - xc[d]);
-                basis.push_back(b);
+                if (std::find(nb_cell, nb_cell + nb, other) != nb_cell + nb) continue;
+                nb_cell[nb] = other;
+                nb_slot[nb] = k;
+                for (int d = 0; d < D; ++d) basis[nb][d] = m.cell_centroid[2 * other + d] - xc[d];
+                ++nb;
             }
         }
-        std::vector<double> ata(D * D, 0.0);
-        for (auto& b : basis)
+        double ata[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int q = 0; q < nb; ++q)
             for (int i = 0; i < D; ++i)
-                for (int j = 0; j < D; ++j) ata[i * D + j] += b[i] * b[j];
-        for (size_t q = 0; q < basis.size(); ++q) {
-            std::vector<double> rhs = basis[q], sys = ata;
-            const bool ok = solve_spd(D, sys, rhs);
-            for (int d = 0; d < D; ++d) p.slot_w[((size_t)nb_slot[q] * 2 + d) * C + c] = ok ? rhs[d] : 0.0;
+                for (int j = 0; j < D; ++j) ata[i * D + j] += basis[q][i] * basis[q][j];
+        for (int q = 0; q < nb; ++q) {
+            const bool ok = solve_spd(D, ata, basis[q]);
+            for (int d = 0; d < D; ++d) p.slot_w[((size_t)nb_slot[q] * 2 + d) * C + c] = ok ? basis[q][d] : 0.0;
         }
         // accumulation order: slots by increasing original face id
         int ks[4] = {0, 1, 2, 3};
