@@ -94,12 +94,14 @@ def peaks():
     return 6650.0, "fallback"
 
 
-def flux_form(launch):
-    """What the kernel kind "flux" is under a launch configuration: the whole
-    stage ("stage"), face + gather ("tile") or the face kernel alone ("face")."""
+def flux_form(launch, profile):
+    """What the kernel kind "flux" was in a profiled run: the whole stage
+    ("stage": no face-state kernel ran; fuse_final alone does not say so, since
+    "mood" at order 1 and tiles too large for shared memory run the separate
+    kernels), face + gather ("tile") or the face kernel alone ("face")."""
     if launch["tile_faces"] <= 0:
         return "face"
-    return "stage" if launch["fuse_final"] else "tile"
+    return "stage" if profile["prep"][1] == 0 else "tile"
 
 
 def algorithmic_bytes(kind, C, F, nq, na, K, stages, form="face"):
@@ -635,7 +637,7 @@ def run_adjoint(a, dev, torch, dist, rank, world):
     C, F = c.mesh.n_cells, c.mesh.n_faces
     g = Solver(c.model, c.mesh, c.settings, p, device=dev)
     tuned = None
-    if not a.no_tune:   # the forward's launch configuration (the replay runs the same kernels)
+    if not a.no_tune:   # the forward's launch configuration (the replays' face knobs stay the handle's own)
         from zoomy_dmplex_b200 import autotune
 
         g.set_state(c.q0)
@@ -880,10 +882,10 @@ def main():
     from zoomy_dmplex_b200.solver import get_launch
 
     launch_cfg = get_launch(g.h)
-    fused = flux_form(launch_cfg)
+    form = flux_form(launch_cfg, prof)
     dom = max((k for k in prof if prof[k][1] > 0), key=lambda k: prof[k][0])
     dom_ms = prof[dom][0] / prof[dom][1]
-    alg = algorithmic_bytes(dom, C, F, nq, na, case.mesh.max_faces, case.settings.ssp_stages, fused)
+    alg = algorithmic_bytes(dom, C, F, nq, na, case.mesh.max_faces, case.settings.ssp_stages, form)
     achieved = alg / (dom_ms / 1e3) / 1e9
     same_cfg = all(launch_cfg.get(k) == v for k, v in NCU_LAUNCH.items())
     traffic = NCU_DRAM_BYTES_PER_CELL.get("%s/%s" % (case.model, dom)) \
@@ -918,12 +920,12 @@ def main():
         peak_tf = pk.value
         s_ = case.settings.ssp_stages
         for k, v in kernel_share.items():
-            fl = fp64_flops(k, case.model, C, F, s_, fused)
+            fl = fp64_flops(k, case.model, C, F, s_, form)
             if fl is not None:
                 v["fp64_tflops"] = fl / (v["ms_per_launch"] / 1e3) / 1e12
         fk = max((k for k in kernel_share if "fp64_tflops" in kernel_share[k]),
                  key=lambda k: kernel_share[k]["share"])
-        fl = fp64_flops(fk, case.model, C, F, s_, fused)
+        fl = fp64_flops(fk, case.model, C, F, s_, form)
         ach = kernel_share[fk]["fp64_tflops"]
         roofline_fp64 = {"bound": "fp64", "kernel": fk, "achieved": ach, "peak": peak_tf, "unit": "TFLOP/s",
                          "frac": ach / peak_tf, "frac_of_unfused": ach / (peak_tf / 2),
