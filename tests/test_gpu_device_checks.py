@@ -1,5 +1,7 @@
 """Device code checked by a small program of its own (compiled here with
-nvcc): the state store for more components than any shipped plugin has."""
+nvcc): the state store for more components than any shipped plugin has, and
+the quotients by a known divisor, whose device form starts from the hardware's
+approximate reciprocal, against the device's own division."""
 import os
 import shutil
 import subprocess
@@ -11,7 +13,8 @@ pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-@pytest.mark.parametrize("name,counts", [("soa_aos_check", {"checked": 364 * 1129})])
+@pytest.mark.parametrize("name,counts", [("soa_aos_check", {"checked": 364 * 1129}),
+                                         ("rn_div_device_check", {"checked": 1 << 26})])
 def test_device_program(tmp_path, name, counts):
     if not shutil.which("nvcc"):
         pytest.fail("nvcc is needed")
