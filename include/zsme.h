@@ -102,7 +102,9 @@ typedef struct zsme_settings {
     int32_t gradient;             /* ZSME_GRADIENT_* */
     int32_t ssp_stages;           /* s of SSP-RK(s,2), >= 2 */
     int32_t source;               /* 1: operator-split implicit source ("splitting") */
-    int32_t block_size;           /* CUDA block size, 0 = library default */
+    int32_t block_size;           /* threads per block of the prep, face and gather kernels, 0 = library
+                                     default; the whole-stage kernel, which a new handle runs instead of
+                                     them, has block sizes of its own */
     int32_t positivity;           /* ZSME_POSITIVITY_* */
     int32_t refresh_derivative_aux; /* solver.refresh_derivative_aux: before every state update, fill the
                                      plugin's derivative aux slots (its field-level update_aux_variables;
@@ -290,11 +292,13 @@ int zsme_batch_get_time(zsme_handle* h, int32_t i, double* t, double* dt);
  * in device memory; 64..1024 runs them as one kernel over tiles of
  * consecutive cells evaluating at most that many faces each, the
  * contributions kept in shared memory (the face block size and cap apply);
- * fuse_final: with tiles (and positivity "none") 1 forms the face states too
- * inside that kernel, a whole stage or right-hand side per launch, with
- * prep_lean 0..1, 2 or 3..4 as 1, 2 or 4 threads per cell and block sizes and
- * caps of its own (the configuration a new handle has); without tiles 1 lets the finalize kernel form the last SSP stage's result
- * itself from the face contributions (separate face and gather kernels,
+ * fuse_final: with tiles 1 forms the face states too inside that kernel, a
+ * whole stage or right-hand side per launch, with prep_lean 0..1, 2 or 3..4 as
+ * 1, 2 or 4 threads per cell (1 with a positivity variant at order 2) and block
+ * sizes and caps of its own (the configuration a new handle has); "mood" at
+ * order 1 and tiles that do not fit its shared memory run the separate kernels
+ * instead; without tiles 1 lets the finalize kernel form the last SSP stage's
+ * result itself from the face contributions (separate face and gather kernels,
  * order 2, positivity other than "mood"), so that result never round-trips
  * through device memory; prep_lean: 1 (default) forms the order-2 face
  * states with the lean kernel (32-bit offsets, branch-free neighbour

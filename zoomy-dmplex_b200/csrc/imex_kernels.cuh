@@ -1,7 +1,7 @@
 // Kernels of the IMEX strategy's step (SolverStrategies.hpp:62-128): the
 // additive Runge-Kutta scheme 2E (imex_tableau.h) with the transport explicit
-// (its right-hand sides G_j come from the ordinary prep / face / gather
-// kernels in MODE_RHS) and the source implicit, solved per cell.  The
+// (its right-hand sides G_j come from the ordinary stage kernels in MODE_RHS)
+// and the source implicit, solved per cell.  The
 // operations are those of the CPU restatement in the same order, so the two
 // agree bit for bit.
 #pragma once

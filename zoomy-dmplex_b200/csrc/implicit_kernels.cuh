@@ -1,7 +1,7 @@
 // Kernels of the fully implicit strategy (SolverStrategies.hpp:133-195): BDF
 // in time, the residual F(t, X, Xdot) = Xdot - S(X) - R(X) of
 // IFunctionWrapper (the transport right-hand side R comes from the ordinary
-// prep / face / gather kernels in MODE_RHS, the source S is the IMEX
+// stage kernels in MODE_RHS, the source S is the IMEX
 // strategy's implicit source), and the preconditioning matrix of
 // ModularSolver::FormImplicitJacobian (ModularSolver.hpp:238-371): per cell
 // a I - dS/dQ (the identity times a in cells drier than 1e-4) plus the
@@ -272,9 +272,10 @@ __global__ void __launch_bounds__(64) imp_cell_jac_kernel(MeshDev m, const doubl
 // LU factors of every diagonal block with partial pivoting (the block-Jacobi
 // preconditioner of the Krylov solve): lu [NQ*NQ][C] with the row swaps of piv
 // [NQ][C], and the reciprocals of the diagonal in rdiag [NQ][C]; a block with a
-// zero or non-finite pivot is applied as the identity.  Every index is known at
-// compile time, so an 8 x 8 block stays in registers, and a column divides by
-// its pivot's reciprocal.
+// zero or non-finite pivot is applied as the identity.  A column divides by its
+// pivot's reciprocal.  The block lives in local memory (a stack frame of its
+// size, 288, 512 and 1152 bytes at 6, 8 and 12 components, no spills): the row
+// swaps' branches keep it out of registers, as gepp_regs.h says of blend.
 template <int NQ>
 __global__ void __launch_bounds__(64) imp_block_lu_kernel(int C, const double* __restrict__ pd,
                                                           double* __restrict__ lu, int* __restrict__ piv,

@@ -1159,7 +1159,7 @@ class Solver final : public SolverBase {
     }
     // The IMEX strategy's transport + source update of one step (SolverStrategies.hpp:62-128,
     // additive Runge-Kutta 2E at the step's dt): G_j = FormRHS(Y_j) by the
-    // prep / face / gather kernels in MODE_RHS, Y_0 = x_ with its implicit
+    // stage kernels in MODE_RHS (launch_rhs), Y_0 = x_ with its implicit
     // source, two implicit stages solved per cell, then x_ updated in place.
     void enqueue_imex_stages(const double* t, const double* dt, const int* act, const double* wl0) {
         namespace K = ark2e;

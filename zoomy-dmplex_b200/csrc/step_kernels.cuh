@@ -5,7 +5,8 @@
 // kernel finds a cell's instance in cell_inst (nullptr: one instance) and
 // takes that instance's parameters, time, dt and activity.
 //
-// One SSP stage = prep_kernel + face_kernel + gather_kernel:
+// One SSP stage = stage_kernel (stage_kernel.cuh), or in separate kernels
+// prep_kernel + face_kernel + gather_kernel:
 //   prep_kernel   per cell: neighbour bounds of the clamped stage state,
 //                 gradient of the unclamped one (least squares or Green-Gauss),
 //                 limited linear reconstruction at each of the cell's faces ->

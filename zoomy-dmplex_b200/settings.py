@@ -9,7 +9,8 @@ default and the gradient the reference's MUSCL path installs,
 ``LeastSquaresGradient`` of ``Gradient.hpp:196-360``, which its MUSCL path
 never installs; its one-sided stencil at reflective walls lets wall cells
 grow without bound under inflow, so it is an option, not the default) and
-``solver.block_size``.
+``solver.block_size`` (threads per block of the separate face-state, face and
+gather kernels; the whole-stage kernel has block sizes of its own).
 
 How the reference interprets the strings, and so how they map here:
 * ``limiter``: only ``"none"`` changes anything; every other value (including
