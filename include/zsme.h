@@ -308,7 +308,8 @@ int zsme_batch_get_time(zsme_handle* h, int32_t i, double* t, double* dt);
  * its register cap takes 4, 6, 8 or none).  Every configuration gives the
  * same results bit for bit.
  * The knobs of the autotuner (zoomy-dmplex_b200/autotune.py).  Setting them
- * outside stream capture only: a new tile_faces rebuilds the tiles. */
+ * outside stream capture only: a new tile_faces rebuilds the tiles; where that
+ * fails (no memory for them) the handle is left with tile_faces 0. */
 int zsme_set_launch(zsme_handle* h, const int32_t* blocks);
 int zsme_get_launch(zsme_handle* h, int32_t* blocks);
 

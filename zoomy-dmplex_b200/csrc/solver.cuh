@@ -251,8 +251,13 @@ class Solver final : public SolverBase {
         }
         imp_drop_graphs();
         adj_drop_graphs();
-        if (ready_) return ensure_tiles();
-        return ZSME_OK;
+        if (!ready_) return ZSME_OK;
+        const int rc = ensure_tiles();
+        if (rc) {   // without its tables (no memory for them) the handle runs the separate kernels
+            lc_.tile_faces = 0;
+            cudaGetLastError();   // the failed allocation's, which the next launch check would report
+        }
+        return rc;
     }
     // (Re)builds the tiles for lc_.tile_faces; outside any stream capture
     // (set-up and zsme_set_launch only).
@@ -294,6 +299,7 @@ class Solver final : public SolverBase {
         if (rc) return rc;
         if (wants_stage() && (rc = upload_stage_tiles(t))) return rc;
         if (tile_built_ == lc_.tile_faces) return ZSME_OK;
+        tile_built_ = 0;   // until every table is there
         ZSME_CUDA(tile_cell_off_.upload(t.cell_off, stream_));
         ZSME_CUDA(tile_face_off_.upload(t.face_off, stream_));
         ZSME_CUDA(tile_in_off_.upload(t.in_off, stream_));
@@ -345,13 +351,16 @@ class Solver final : public SolverBase {
         StageTiles s;
         int rc = build_stage_tiles(pm_, t, st_.reconstruction_order, st_.gradient != ZSME_GRADIENT_LSQ, s);
         if (rc) return rc;
-        st_built_ = lc_.tile_faces;
+        st_built_ = 0;   // until every table is there
         st_fst_ = t.max_faces + 1;
         st_cst_ = s.max_local;
         size_t smem = 0;
         for (int p : {1, 2, 4}) smem = std::max(smem, stage_smem(p));
         st_fits_ = s.fits && smem <= kMaxStageSmem;
-        if (!st_fits_) return ZSME_OK;   // the separate stage kernels run instead
+        if (!st_fits_) {   // the separate stage kernels run instead
+            st_built_ = lc_.tile_faces;
+            return ZSME_OK;
+        }
         auto up = [&](DevBuf<int>& d, std::vector<int>& v) {
             if (v.empty()) v.push_back(0);
             return d.upload(v, stream_);
@@ -383,6 +392,7 @@ class Solver final : public SolverBase {
                                                        st_.gradient == ZSME_GRADIENT_LSQ, st_geo_.p);
         ZSME_CUDA(cudaGetLastError());
         ZSME_CUDA(cudaStreamSynchronize(stream_));   // a chained launch reads it without waiting for the stream
+        st_built_ = lc_.tile_faces;
         return ZSME_OK;
     }
     int stage_row(int parts, int n) const {
